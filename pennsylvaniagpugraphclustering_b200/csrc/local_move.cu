@@ -1909,8 +1909,10 @@ struct Mover {
                 PGGC_LAUNCH_CHECK();
             } else {
                 const bool split = !strict && ord.n_huge > 0 && ord.n_huge <= 65535;
+                // without k_mark_huge every row is marked here, also one of more
+                // than n edges (parallel edges)
                 k_mark_affected<W><<<grid_for(ctx, ceil_div(nm, 8), 1, 16), 256, 0, ctx.stream>>>(
-                    gv, moves.p, nm, flags.p, split ? HUGE_DEG : n);
+                    gv, moves.p, nm, flags.p, split ? HUGE_DEG : g.nnz);
                 PGGC_LAUNCH_CHECK();
                 if (split) {
                     k_mark_huge<W><<<dim3((unsigned)ceil_div(ord.max_deg, MARK_CHUNK), (unsigned)ord.n_huge), 512, 0,

@@ -6,6 +6,7 @@ import pytest
 
 import pennsylvaniagpugraphclustering_b200 as pg
 from pennsylvaniagpugraphclustering_b200 import _lib
+from pennsylvaniagpugraphclustering_b200 import move_filter as MF
 
 pytestmark = pytest.mark.gpu
 
@@ -152,3 +153,35 @@ def test_float_tables_in_units(mem, kind, n):
     moves = (best >= np.maximum(own.astype(np.float32), 0)) & np.isfinite(best)
     assert np.array_equal(dest >= 0, moves)
     assert np.array_equal(gain[moves], (best[moves].astype(np.float32) - own[moves].astype(np.float32)))
+
+
+@pytest.mark.parametrize("weights", [False, True])
+@pytest.mark.parametrize("how", ["strict", "logging"])
+def test_rows_of_more_edges_than_vertices(mem, how, weights):
+    """Parallel edges: 80 triples a - b - c in 1,000 vertices, 1,100 edges from a to b and 1,200 from b to c.  From
+    {a}, {b, c} every a moves; its neighbour b gains that row in own-cluster weight, and the objective kept by the
+    sweeps must be the labels' own.  Few enough movers for their rows to be pushed, enough for the flags."""
+    n, k, ab, bc = 1000, 80, 1100, 1200
+    a = 3 * np.arange(k, dtype=np.int32)
+    src = np.concatenate([np.repeat(a, ab), np.repeat(a + 1, bc)])
+    dst = src + 1
+    w = (1 + np.arange(len(src)) % 3).astype(np.int32) if weights else None
+    objective = pg.OBJ_WMOD if weights else pg.OBJ_MOD
+    g = pg.graph_from_edges(mem, n, src, dst, w, symmetric=True, objective=objective)
+    assert np.diff(g.to_host()[0]).max() > n
+    part = np.arange(n, dtype=np.int32)
+    part[a + 2] = a + 1
+    rfd = pg.get_objective(mem, g, objective)
+    td = np.zeros(n, np.int64)
+    np.add.at(td, part, g.to_host()[3])
+    rfd.set_state(n, td, 2.0 * (np.ones(len(src)) if w is None else w)[k * ab:].sum())
+    if how == "strict":
+        st = pg.local_move_strict(mem, g, part, rfd, False)
+    else:
+        MF.log_start(mem, 1 << 16)
+        try:
+            st = pg.local_move(mem, g, part, rfd, False, enable_simulated_annealing=False)
+        finally:
+            MF.log_stop(mem, 1 << 16)
+    assert st["moves"] == k and np.array_equal(part[a], part[a + 1]) and np.array_equal(part[a], part[a + 2])
+    assert rfd.get_objective() == pytest.approx(pg.verify_objective(mem, g, part, objective)[0], rel=1e-12)
