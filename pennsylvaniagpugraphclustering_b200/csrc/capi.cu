@@ -243,6 +243,7 @@ std::unique_ptr<Graph<W>> make_graph(Context& ctx, int64_t n, int64_t nnz, const
     }
     row_sums<W>(ctx, *g);
     ctx.sync();
+    g->cache->sums.clear();
     return g;
 }
 
@@ -261,6 +262,7 @@ std::unique_ptr<Graph<i32>> adopt_graph(Context& ctx, i64 n, i64 nnz, DBuf<i64>&
     default_vertex_weights<i32>(ctx, *g, objective);
     row_sums<i32>(ctx, *g);
     ctx.sync();
+    g->cache->sums.clear();
     return g;
 }
 

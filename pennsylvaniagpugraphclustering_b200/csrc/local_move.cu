@@ -1458,39 +1458,47 @@ __global__ void k_row_degrees(const i64* rowptr, i64 n, V* out) {
         out[i] = V(rowptr[i + 1] - rowptr[i]);
 }
 
-// graphs are created with their sums (make_graph) or by one context (coarse
-// levels); the lock covers a graph first used by several threads
-static std::mutex g_graph_cache_mu;
-
+// Kept with the graph.  The kernels that fill them are queued and not waited
+// for: a coarse graph may get its sums from one of several jobs that share it,
+// so a call on another stream waits for the mark that the first one left.
+// (The units are values that tables are built on: read too early they turn
+// fractional weights into whole numbers.)
 template <class W>
 const typename Traits<W>::V* row_sums(Context& ctx, const Graph<W>& g) {
     using V = typename Traits<W>::V;
     if (g.n == 0) return nullptr;
-    std::lock_guard<std::mutex> lk(g_graph_cache_mu);
-    if (!g.rsum.p) {
-        g.rsum = DBuf<V>(ctx, g.n);
-        const int grid = (int)std::min<i64>(ceil_div(g.n, 32), (i64)ctx.num_sms * 16);
-        if (g.uniform) {
-            k_row_degrees<V><<<grid, 256, 0, ctx.stream>>>(g.view().rowptr, g.n, g.rsum.p);
+    GraphCache& c = *g.cache;
+    std::lock_guard<std::mutex> lk(c.mu);
+    if (g.rsum.p) {
+        c.sums.wait(ctx);
+        return g.rsum.p;
+    }
+    DBuf<V> sums(ctx, g.n);
+    DBuf<WeightUnits> units;
+    const int grid = (int)std::min<i64>(ceil_div(g.n, 32), (i64)ctx.num_sms * 16);
+    if (g.uniform) {
+        k_row_degrees<V><<<grid, 256, 0, ctx.stream>>>(g.view().rowptr, g.n, sums.p);
+        PGGC_LAUNCH_CHECK();
+    } else {
+        const i64 most = g.nnz / ROW_SUM_BIG;  // rows above it
+        Tmp<unsigned long long> nbig(ctx, 1);
+        Tmp<i32> big(ctx, most + 1);
+        PGGC_CUDA(cudaMemsetAsync(nbig.p, 0, sizeof(unsigned long long), ctx.stream));
+        if (std::is_same<V, double>::value) {
+            units = DBuf<WeightUnits>(ctx, 1);
+            PGGC_CUDA(cudaMemsetAsync(units.p, 0, sizeof(WeightUnits), ctx.stream));
+        }
+        k_row_sums<W><<<grid, 256, 0, ctx.stream>>>(g.view(), sums.p, big.p, nbig.p, units.p);
+        PGGC_LAUNCH_CHECK();
+        if (most > 0) {
+            k_row_sums_big<W><<<(int)std::min<i64>(most, (i64)ctx.num_sms * 2), 1024, 0, ctx.stream>>>(
+                g.view(), sums.p, big.p, nbig.p, units.p);
             PGGC_LAUNCH_CHECK();
-        } else {
-            const i64 most = g.nnz / ROW_SUM_BIG;  // rows above it
-            Tmp<unsigned long long> nbig(ctx, 1);
-            Tmp<i32> big(ctx, most + 1);
-            PGGC_CUDA(cudaMemsetAsync(nbig.p, 0, sizeof(unsigned long long), ctx.stream));
-            if (std::is_same<V, double>::value) {
-                g.units = DBuf<WeightUnits>(ctx, 1);
-                PGGC_CUDA(cudaMemsetAsync(g.units.p, 0, sizeof(WeightUnits), ctx.stream));
-            }
-            k_row_sums<W><<<grid, 256, 0, ctx.stream>>>(g.view(), g.rsum.p, big.p, nbig.p, g.units.p);
-            PGGC_LAUNCH_CHECK();
-            if (most > 0) {
-                k_row_sums_big<W><<<(int)std::min<i64>(most, (i64)ctx.num_sms * 2), 1024, 0, ctx.stream>>>(
-                    g.view(), g.rsum.p, big.p, nbig.p, g.units.p);
-                PGGC_LAUNCH_CHECK();
-            }
         }
     }
+    c.sums.set(ctx);
+    g.units = std::move(units);
+    g.rsum = std::move(sums);
     return g.rsum.p;
 }
 

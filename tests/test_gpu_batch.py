@@ -116,3 +116,24 @@ def test_autotuner_picks_the_fastest_trial_and_keeps_results(mem):
             assert st["objective"] == so["objective"]
     finally:
         pg.tune_set(mem, **{k: saved[k] for k in ("thread_max_deg", "warp_max_deg", "load_factor", "streams")})
+
+
+@pytest.mark.parametrize("weights", ["float", "unit"])
+def test_jobs_share_a_coarse_graph_without_sums(mem, weights):
+    """A large coarse graph comes without row sums and weight units: one job of the batch fills them while the others
+    start on it, and every job still gets the sequential run's labels."""
+    hg = gg.dcsbm(150000, 4, mean_deg=16)
+    obj = pg.OBJ_WMOD if weights == "float" else pg.OBJ_MOD
+    g = pg.weighted_graph(mem, hg.rowptr, hg.col, hg.w if weights == "float" else None, objective=obj)
+    nc = 60000
+    vcmap = np.random.default_rng(1).permutation(np.arange(g.n) % nc).astype(np.int32)
+    coarse = pg.build_coarse_graph(mem, g, vcmap, nc)
+    seeds = [1, 2, 3, 4, 5, 6]
+    want = [_seq(mem, coarse, obj, pg.METHOD_LEIDEN_PLUS, 0, s) for s in seeds]
+    for _ in range(4):
+        fresh = pg.build_coarse_graph(mem, g, vcmap, nc)
+        got = pg.batch_run(mem, [dict(graph=fresh, objective=obj, method=pg.METHOD_LEIDEN_PLUS, ex_iters=0, seed=s)
+                                 for s in seeds], streams=len(seeds))
+        for (lab, st), (lo, so) in zip(got, want):
+            assert np.array_equal(lab, lo) and st["objective"] == so["objective"]
+        fresh.close()
