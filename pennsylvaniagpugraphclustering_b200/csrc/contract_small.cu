@@ -2,7 +2,7 @@
 //
 // The general contraction (contract.cu) is about 25 launches and two host
 // round trips, 120-140 us however small the graph.  For the graphs that
-// lm_small.cu moves, one cluster does all of it, and the products the next
+// lm_cluster.cuh moves, one cluster does all of it, and the products the next
 // level starts with: the degree ordering, the class lists and the row sums
 // (12 launches and two round trips of their own).
 //

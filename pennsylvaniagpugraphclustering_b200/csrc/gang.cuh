@@ -1,6 +1,6 @@
 // gang.cuh -- steps run by all blocks of one thread-block cluster.
 //
-// The kernels for small graphs (lm_small.cu, contract_small.cu, ...) run a
+// The kernels for small graphs (lm_cluster.cuh, contract_small.cu, ...) run a
 // whole sequence of steps in one launch of a single cluster, "the gang": the
 // steps loop over their items with the gang's threads or warps and are
 // separated by gang_sync().

@@ -1,4 +1,4 @@
-// lm_small.cuh -- local moves of small graphs in one launch (lm_small.cu).
+// lm_small.cuh -- local moves of small graphs in one launch (lm_cluster.cuh).
 #pragma once
 #include "filter.cuh"
 #include "gang.cuh"
@@ -57,7 +57,7 @@ struct SmallArgs {
 };
 
 // The same steps launched one by one over the whole GPU, for graphs above the
-// one-launch size (lm_small.cu).
+// one-launch size (lm_steps.cu).
 template <class W>
 void step_init(Context& ctx, const SmallArgs<W>& a);  // current state <- best state
 template <class W>

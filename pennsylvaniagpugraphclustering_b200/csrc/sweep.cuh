@@ -2,7 +2,7 @@
 // scalars, the DeltaQ argmax of one vertex, hash-table inserts and the
 // afterburner term (src/local_mover.cpp:280-634).  Included by the kernels of
 // local_move.cu (one kernel per degree class, every graph size) and by
-// lm_small.cu (a whole local move in one launch, small graphs).
+// lm_steps.cuh (one-launch local moves of small graphs, a launch per step above).
 #pragma once
 #include "kernels.cuh"
 
