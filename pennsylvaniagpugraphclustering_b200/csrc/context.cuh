@@ -361,6 +361,11 @@ struct DBuf {
     i64 n = 0;
     DBuf() = default;
     DBuf(Context& c, i64 count) : ctx(&c), p(c.alloc<T>(count)), n(count) {}
+    // a buffer of `home`, allocated in the order of c's stream: home's pool
+    // gives it and home's stream takes it back, so it may outlive c
+    DBuf(Context& home, Context& c, i64 count) : ctx(&home), n(count) {
+        PGGC_CUDA(cudaMallocFromPoolAsync((void**)&p, sizeof(T) * (size_t)(count > 0 ? count : 1), home.pool, c.stream));
+    }
     DBuf(DBuf&& o) noexcept : ctx(o.ctx), p(o.p), n(o.n) {
         o.p = nullptr;
         o.n = 0;

@@ -189,9 +189,9 @@ ClassLists graph_class_lists(Context& ctx, const Graph<W>& g, const Ordering& or
     std::lock_guard<std::mutex> lk(c.mu);
     ClassLists cl;
     if (!c.cls_ok) {
-        c.cls_list = DBuf<i32>(ctx, std::max<i64>(ord.n, 1));
-        c.cls_off = DBuf<i64>(ctx, NCLS + 1);
-        c.cls_cnt = DBuf<unsigned long long>(ctx, 2 * NCLS);
+        c.cls_list = g.template kept<i32>(ctx, std::max<i64>(ord.n, 1));
+        c.cls_off = g.template kept<i64>(ctx, NCLS + 1);
+        c.cls_cnt = g.template kept<unsigned long long>(ctx, 2 * NCLS);
         cl.list = c.cls_list.p;
         cl.off = c.cls_off.p;
         cl.cnt = c.cls_cnt.p;
@@ -1473,7 +1473,7 @@ const typename Traits<W>::V* row_sums(Context& ctx, const Graph<W>& g) {
         c.sums.wait(ctx);
         return g.rsum.p;
     }
-    DBuf<V> sums(ctx, g.n);
+    DBuf<V> sums = g.template kept<V>(ctx, g.n);
     DBuf<WeightUnits> units;
     const int grid = (int)std::min<i64>(ceil_div(g.n, 32), (i64)ctx.num_sms * 16);
     if (g.uniform) {
@@ -1485,7 +1485,7 @@ const typename Traits<W>::V* row_sums(Context& ctx, const Graph<W>& g) {
         Tmp<i32> big(ctx, most + 1);
         PGGC_CUDA(cudaMemsetAsync(nbig.p, 0, sizeof(unsigned long long), ctx.stream));
         if (std::is_same<V, double>::value) {
-            units = DBuf<WeightUnits>(ctx, 1);
+            units = g.template kept<WeightUnits>(ctx, 1);
             PGGC_CUDA(cudaMemsetAsync(units.p, 0, sizeof(WeightUnits), ctx.stream));
         }
         k_row_sums<W><<<grid, 256, 0, ctx.stream>>>(g.view(), sums.p, big.p, nbig.p, units.p);

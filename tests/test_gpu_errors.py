@@ -7,6 +7,7 @@ import pytest
 
 import pennsylvaniagpugraphclustering_b200 as pg
 from pennsylvaniagpugraphclustering_b200 import _lib
+from pennsylvaniagpugraphclustering_b200 import graphgen as gg
 
 from . import graphs as G
 
@@ -78,3 +79,39 @@ def test_destruction_order_is_free(mem):
     m2.close()  # the C context stays alive while wg and cd reference it
     cd.close()
     wg.close()
+
+
+@pytest.mark.parametrize("coarse", [False, True])
+def test_graph_outlives_a_context_that_worked_on_it(mem, coarse):
+    """What calls on another context add to a graph (ordering, class lists, row sums and units) stays with the graph
+    when that context is gone, and is freed with the graph."""
+    hg = gg.dcsbm(90000, 3, mean_deg=12)
+    owner = pg.memory_store(0)
+    g = pg.weighted_graph(owner, hg.rowptr, hg.col, hg.w, objective=pg.OBJ_WMOD)
+    if coarse:  # without row sums
+        vcmap = (np.arange(g.n) % 45000).astype(np.int32)
+        g = pg.build_coarse_graph(owner, g, vcmap, 45000)
+
+    def work(store):
+        rfd = pg.get_objective(store, g, pg.OBJ_WMOD)
+        part = np.arange(g.n, dtype=np.int32)
+        pg.local_move(store, g, part, rfd, True)
+        vc, nc = pg.coarsen_leidenR(store, g, part, rfd, 1, 2)
+        nxt = pg.build_coarse_graph(store, g, vc, nc)
+        out = part, vc, nc, rfd.obj, nxt.to_host()[2]
+        nxt.close()
+        rfd.close()
+        return out
+
+    visitor = pg.memory_store(0)
+    first = work(visitor)
+    visitor.close()
+    others = [pg.memory_store(0) for _ in range(3)]  # host and device memory of the closed context is taken again
+    second = work(owner)
+    for a, b in zip(first, second):
+        assert np.array_equal(a, b)
+    g.close()
+    for store in others:
+        store.close()
+    h = pg.weighted_graph(owner, hg.rowptr, hg.col, hg.w, objective=pg.OBJ_WMOD)
+    pg.run_clustering(owner, h, pg.get_objective(owner, h, pg.OBJ_WMOD), method=pg.METHOD_LEIDEN)
