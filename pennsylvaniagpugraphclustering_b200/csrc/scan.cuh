@@ -290,13 +290,15 @@ void sum_i64(Context& ctx, In in, i64 k, i64* d_out) {
 // with a count per 512-key warp tile, in 64 bits, the counts of a 33 M-key
 // sort were 134 MB a pass, read and written three times, and the keys went out
 // one by one; 33 M keys of 40 bits took 13 ms.  Bound by memory traffic now
-// (two reads and one write of the keys a pass).
+// (two reads and one write of the keys a pass).  O: places of the keys, 32-bit
+// where they fit.
 constexpr int RS_THREADS = 512;
 constexpr int RS_WARPS = RS_THREADS / 32;
 constexpr int RS_ITEMS = 8;
 constexpr i64 RS_TILE = RS_THREADS * RS_ITEMS;
 
-static __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const u64* keys, i64 k, int shift, i64 ntiles, u32* hist) {
+template <class O>
+__global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const u64* keys, i64 k, int shift, i64 ntiles, O* hist) {
     __shared__ u32 cnt[RS_WARPS][256];
     const int w = threadIdx.x >> 5, l = lane_id();
     for (int d = l; d < 256; d += 32) cnt[w][d] = 0;
@@ -318,12 +320,13 @@ static __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const u64* keys, 
 
 struct NoPayload {};
 
-template <class P>
+template <class P, class O>
 __global__ void __launch_bounds__(RS_THREADS, 2) k_rs_scatter(const u64* keys, const P* vals, u64* keys_out, P* vals_out,
-                                                              i64 k, int shift, i64 ntiles, const u32* off) {
+                                                              i64 k, int shift, i64 ntiles, const O* off) {
     constexpr bool HAS = !std::is_same<P, NoPayload>::value;
     __shared__ unsigned short cnt[RS_WARPS][256];  // at most a tile's 4,096
-    __shared__ u32 start[256], gbase[256], wsum[8];
+    __shared__ u32 start[256], wsum[8];
+    __shared__ O gbase[256];  // modulo the type: place minus position in the tile
     __shared__ __align__(16) u64 buf[RS_TILE];
     const int w = threadIdx.x >> 5, l = lane_id();
     for (int d = l; d < 256; d += 32) cnt[w][d] = 0;
@@ -382,13 +385,13 @@ __global__ void __launch_bounds__(RS_THREADS, 2) k_rs_scatter(const u64* keys, c
         buf[pos[it]] = key[it];
     }
     __syncthreads();
-    u32 to[RS_ITEMS];
+    O to[RS_ITEMS];
 #pragma unroll
     for (int it = 0; it < RS_ITEMS; it++) {
         const int i = it * RS_THREADS + threadIdx.x;
         if (i < count) {
             const u64 x = buf[i];
-            to[it] = gbase[(x >> shift) & 255] + (u32)i;
+            to[it] = gbase[(x >> shift) & 255] + (O)i;
             keys_out[to[it]] = x;
         }
     }
@@ -410,34 +413,30 @@ __global__ void __launch_bounds__(RS_THREADS, 2) k_rs_scatter(const u64* keys, c
     }
 }
 
-struct ArrIn32 {
-    const u32* a;
+template <class O>
+struct PlaceIn {
+    const O* a;
     __device__ i64 operator()(i64 i) const { return (i64)a[i]; }
 };
-struct ArrOutExcl32 {
-    u32* a;
-    __device__ void operator()(i64 i, i64 excl, i64) const { a[i] = (u32)excl; }
+template <class O>
+struct PlaceOut {
+    O* a;
+    __device__ void operator()(i64 i, i64 excl, i64) const { a[i] = (O)excl; }
 };
 
-// Sorts keys[0..k) (with payload vals unless P is NoPayload) on bits
-// [begin_bit, end_bit).  Uses the provided temporaries; the result is left in
-// keys/vals.
-template <class P>
-void radix_sort_pairs(Context& ctx, u64* keys, P* vals, i64 k, int begin_bit, int end_bit, u64* keys_tmp,
-                      P* vals_tmp) {
+template <class P, class O>
+void radix_sort_places(Context& ctx, u64* keys, P* vals, i64 k, int begin_bit, int end_bit, u64* keys_tmp, P* vals_tmp) {
     constexpr bool HAS = !std::is_same<P, NoPayload>::value;
-    if (k <= 1) return;
-    if (k > 0xFFFFFFFFll) throw InvalidArg("radix sort of more than 2^32 - 1 keys");
     i64 ntiles = ceil_div(k, RS_TILE);
-    Tmp<u32> hist(ctx, 256 * ntiles);
+    Tmp<O> hist(ctx, 256 * ntiles);
     u64 *ka = keys, *kb = keys_tmp;
     P *va = vals, *vb = vals_tmp;
     int passes = 0;
     for (int shift = begin_bit; shift < end_bit; shift += 8) {
-        k_rs_hist<<<(unsigned)ntiles, RS_THREADS, 0, ctx.stream>>>(ka, k, shift, ntiles, hist.p);
+        k_rs_hist<O><<<(unsigned)ntiles, RS_THREADS, 0, ctx.stream>>>(ka, k, shift, ntiles, hist.p);
         PGGC_LAUNCH_CHECK();
-        scan_apply(ctx, ArrIn32{hist.p}, ArrOutExcl32{hist.p}, 256 * ntiles, nullptr, nullptr);
-        k_rs_scatter<P><<<(unsigned)ntiles, RS_THREADS, 0, ctx.stream>>>(ka, va, kb, vb, k, shift, ntiles, hist.p);
+        scan_apply(ctx, PlaceIn<O>{hist.p}, PlaceOut<O>{hist.p}, 256 * ntiles, nullptr, nullptr);
+        k_rs_scatter<P, O><<<(unsigned)ntiles, RS_THREADS, 0, ctx.stream>>>(ka, va, kb, vb, k, shift, ntiles, hist.p);
         PGGC_LAUNCH_CHECK();
         std::swap(ka, kb);
         std::swap(va, vb);
@@ -447,6 +446,17 @@ void radix_sort_pairs(Context& ctx, u64* keys, P* vals, i64 k, int begin_bit, in
         copy_d2d(ctx, keys, ka, k);
         if constexpr (HAS) copy_d2d(ctx, vals, va, k);
     }
+}
+
+// Sorts keys[0..k) (with payload vals unless P is NoPayload) on bits
+// [begin_bit, end_bit).  Uses the provided temporaries; the result is left in
+// keys/vals.
+template <class P>
+void radix_sort_pairs(Context& ctx, u64* keys, P* vals, i64 k, int begin_bit, int end_bit, u64* keys_tmp,
+                      P* vals_tmp) {
+    if (k <= 1) return;
+    if (k <= 0xFFFFFFFFll) radix_sort_places<P, u32>(ctx, keys, vals, k, begin_bit, end_bit, keys_tmp, vals_tmp);
+    else radix_sort_places<P, u64>(ctx, keys, vals, k, begin_bit, end_bit, keys_tmp, vals_tmp);
 }
 
 inline int bits_for(u64 maxval) {

@@ -234,3 +234,42 @@ def test_edges_at_sort_tile_edges(mem, n, m, weighted):
     assert np.array_equal(col, v[order])
     if weighted:
         assert np.array_equal(ww, np.repeat(w[keep], 2)[order])
+
+
+def test_edge_lists_of_more_than_2_31_pairs():
+    """2^32 + 2^20 sort keys, so 64-bit places: a repeated block of pairs that deduplicates to a known set, and a path
+    above it whose keys sort last, half of them beyond 2^32, once each.  About 105 GB on the device."""
+    torch = pytest.importorskip("torch")
+    if torch.cuda.mem_get_info()[0] < 130 << 30:
+        pytest.skip("needs 130 GB of free device memory")
+    low, n = 2048, 1 << 20
+    path = n - 1 - low  # pairs (u, u + 1), u >= low, spread over the list's start
+    m = (1 << 31) - (1 << 19) + path
+    k = 2 * m
+    assert k > 1 << 32 and k - 2 * path < 1 << 32
+    src = torch.empty(m, dtype=torch.int32, device="cuda")
+    dst = torch.empty(m, dtype=torch.int32, device="cuda")
+    src[:path] = torch.arange(low, n - 1, device="cuda", dtype=torch.int32)
+    dst[:path] = src[:path] + 1
+    for a in range(path, m, 1 << 27):
+        j = torch.arange(a, min(m, a + (1 << 27)), device="cuda")
+        u = j % low
+        src[a:a + (1 << 27)] = u
+        dst[a:a + (1 << 27)] = (u + 1 + 3 * (j // low % 300)) % low  # differences 1, 4, ... 898
+        del j, u
+    store = pg.memory_store(0)  # its pool is given back at the end
+    try:
+        g = pg.graph_from_edges(store, n, src, dst, symmetric=False)
+        rowptr, col, _, _ = g.to_host()
+        g.close()
+    finally:
+        store.close()
+        del src, dst
+        torch.cuda.empty_cache()
+    u = np.arange(low)[:, None]
+    d = 1 + 3 * np.arange(300)[None, :]
+    a, b = np.broadcast_to(u, (low, 300)).ravel(), ((u + d) % low).ravel()
+    p = np.arange(low, n - 1)
+    key = np.unique(np.concatenate([a * n + b, b * n + a, p * n + p + 1, (p + 1) * n + p]))
+    assert np.array_equal(rowptr, np.concatenate([[0], np.cumsum(np.bincount(key // n, minlength=n))]))
+    assert np.array_equal(col, key % n)
