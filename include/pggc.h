@@ -89,6 +89,11 @@ uint64_t pggc_launch_count(void);
  * context stays usable. */
 pggc_status pggc_debug_set_probe_limit(pggc_context* ctx, int limit);
 
+/* For tests: take the device to place no thread-block cluster of more than
+ * `blocks` blocks (16 restores the default), as a partition of a GPU may.
+ * Results do not depend on it. */
+pggc_status pggc_debug_set_cluster_limit(pggc_context* ctx, int blocks);
+
 /* Per-kernel-family timing (CUDA events on the context stream) and algorithmic
  * byte counts, for roofline reporting; the counterpart of the reference's
  * EXTRA_TIMING measurements (src/clustering_methods.cpp:78-108).  Families:

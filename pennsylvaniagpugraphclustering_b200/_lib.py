@@ -80,6 +80,7 @@ _SIGS = {
     "pggc_version": (ctypes.c_char_p, []),
     "pggc_launch_count": (_u64, []),
     "pggc_debug_set_probe_limit": (_ci, [_vp, _ci]),
+    "pggc_debug_set_cluster_limit": (_ci, [_vp, _ci]),
     "pggc_profile_enable": (_ci, [_vp, _ci]),
     "pggc_profile_reset": (_ci, [_vp]),
     "pggc_profile_names": (_ci, [_vp, ctypes.c_char_p, _i64, ctypes.POINTER(_i64)]),

@@ -335,6 +335,14 @@ pggc_status pggc_debug_set_probe_limit(pggc_context* ctx, int limit) {
     });
 }
 
+pggc_status pggc_debug_set_cluster_limit(pggc_context* ctx, int blocks) {
+    return guarded([&] {
+        need(ctx != nullptr, "NULL context");
+        need(blocks >= 0 && blocks <= 16, "blocks must be in [0, 16]");
+        ctx->ctx->max_cluster = blocks;
+    });
+}
+
 pggc_status pggc_profile_enable(pggc_context* ctx, int on) {
     return guarded([&] {
         need(ctx != nullptr, "NULL context");
@@ -949,6 +957,7 @@ static void batch_impl(pggc_context* ctx, pggc_batch_job* jobs, int64_t count, i
         // the main context's kernel knobs and learned filter (network,
         // threshold, counters) are shared read-only
         wc.tune = c.tune;
+        wc.max_cluster = c.max_cluster;
         wc.filt.mode = c.filt.mode;
         wc.filt.net = c.filt.net;
         wc.filt.threshold = c.filt.threshold;

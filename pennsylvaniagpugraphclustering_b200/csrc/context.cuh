@@ -49,6 +49,9 @@ struct Context {
     size_t max_smem_optin = 0;
     // fault injection: cap on hash-table probes (0 = only the table size bounds them)
     u32 probe_cap = 0;
+    // and on the blocks of a cluster, as on a partition of the GPU that places
+    // no larger one
+    int max_cluster = 16;
     // profiling
     bool profiling = false;
     unsigned long long* d_prof = nullptr;  // [64] device byte counters

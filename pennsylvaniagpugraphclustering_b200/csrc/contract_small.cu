@@ -412,8 +412,9 @@ template <class W>
 std::unique_ptr<Graph<W>> build_coarse_small(Context& ctx, const Graph<W>& g, const i32* vcmap, i64 nc) {
     using V = typename Traits<W>::V;
     const i64 n = g.n, nnz = g.nnz;
-    const int blocks = small_cluster_blocks(n, nnz);
-    if (blocks == 0 || nc == 0 || n == 0 || ctx.probe_cap != 0) return nullptr;
+    if (nc == 0 || n == 0 || ctx.probe_cap != 0) return nullptr;
+    const int blocks = gang_blocks(ctx, k_contract_small<W>, small_cluster_blocks(n, nnz));
+    if (blocks == 0) return nullptr;
     ProfScope ps(ctx, "contract_small");
     const bool matrix = nc <= CS_MATRIX_NC;
     const i64 room = std::max<i64>(std::min<i64>(nnz, nc * (nc - 1)), 1);

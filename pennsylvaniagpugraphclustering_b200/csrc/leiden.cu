@@ -1046,8 +1046,9 @@ i64 refine_small(Context& ctx, const Graph<W>& g, const Ordering& ord, const i32
                  bool reuse) {
     using V = typename Traits<W>::V;
     const i64 n = g.n;
-    const int blocks = small_cluster_blocks(n, g.nnz);
-    if (blocks == 0 || ord.off_large2 < n || ctx.probe_cap != 0) return -1;
+    if (ord.off_large2 < n || ctx.probe_cap != 0) return -1;
+    const int blocks = gang_blocks(ctx, k_refine_small<W>, small_cluster_blocks(n, g.nnz));
+    if (blocks == 0) return -1;
     const ClassLists cls = graph_class_lists<W>(ctx, g, ord);
     RefineArgs<W> a{};
     a.g = g.view();

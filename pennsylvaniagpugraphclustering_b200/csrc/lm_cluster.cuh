@@ -204,15 +204,20 @@ bool local_move_small(Context& ctx, const Graph<W>& g, const Ordering& ord, i32*
     using V = typename Traits<W>::V;
     const i64 n = g.n;
     const bool long_rows = g.nnz >= 64 * n;
-    const int blocks = g.nnz > (long_rows ? LS_MOVE_NNZ_LONG : LS_MOVE_NNZ) ? 0 : small_cluster_blocks(n, g.nnz);
+    const int want = g.nnz > (long_rows ? LS_MOVE_NNZ_LONG : LS_MOVE_NNZ) ? 0 : small_cluster_blocks(n, g.nnz);
     auto& F = ctx.filt;
     const bool filt_on = F.mode != 0 && !strict;
     const bool gating = F.mode == 2 && !strict && !F.suspended && F.level >= F.min_level &&
                         !(F.max_pass >= 0 && F.pass >= F.max_pass);
     // logging runs, rows summed by 1024 threads and injected probe faults keep the general path
-    if (blocks == 0 || F.mode == 1 || (gating && constrained) || ord.off_large2 < n || ctx.probe_cap != 0 ||
+    if (want == 0 || F.mode == 1 || (gating && constrained) || ord.off_large2 < n || ctx.probe_cap != 0 ||
         best.label_count > LS_MAX_LABELS || (strict && sweep_limit == 0))
         return false;
+    const auto kern = gating        ? k_local_move_small<W, false, true>
+                      : constrained ? k_local_move_small<W, true, false>
+                                    : k_local_move_small<W, false, false>;
+    const int blocks = gang_blocks(ctx, kern, want);
+    if (blocks == 0) return false;
     ProfScope ps(ctx, "local_move_small");
     const ClassLists cls = graph_class_lists<W>(ctx, g, ord);
     // labels that the sweeps can reach: each appends at most one per vertex
@@ -281,12 +286,8 @@ bool local_move_small(Context& ctx, const Graph<W>& g, const Ordering& ord, i32*
         f.net = F.net;
         f.threshold = F.threshold;
         f.stats = F.stats;
-        launch_gang(ctx, k_local_move_small<W, false, true>, a, blocks);
-    } else if (constrained) {
-        launch_gang(ctx, k_local_move_small<W, true, false>, a, blocks);
-    } else {
-        launch_gang(ctx, k_local_move_small<W, false, false>, a, blocks);
     }
+    launch_gang(ctx, kern, a, blocks);
     const LMScalars<V>* h = (const LMScalars<V>*)ctx.readback(a.sc, sizeof(LMScalars<V>));
     if (h->num_cand != 0) {  // strict, with candidates: the retained weights still stand
         ctx.pv_uid = pv_uid;

@@ -77,7 +77,7 @@ void step_sums(Context& ctx, const SmallArgs<W>& a);
 template <class W>
 void step_objective(Context& ctx, const SmallArgs<W>& a, bool sweep, i64 label_bound);
 
-// Blocks of the cluster that runs a step of this graph, 0 when it is not small.
+// Blocks of the cluster that should run a step of this graph, 0 when it is not small.
 int small_cluster_blocks(i64 n, i64 nnz);
 
 // local_move or local_move_strict of a small graph; false, with nothing done,
@@ -97,36 +97,64 @@ enum ContractSmallSlot : int {
     CSS_OVAL = 110, CSS_UCOUNT, CSS_FIXED, CSS_PRES, CSS_OKEY, CSS_CNT, CSS_CSTART, CSS_P, CSS_MEMBERS, CSS_BIG
 };
 
-// Allows clusters of up to 16 blocks for `kernel`, once per (kernel, device).
-template <class K>
-inline void set_wide_clusters_once(K kernel, int device) {
+// The cluster launch of `kern` with `blocks` blocks.
+struct GangLaunch {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at[1];
+    GangLaunch(int blocks, cudaStream_t stream) {
+        cfg.gridDim = dim3(blocks);
+        cfg.blockDim = dim3(LS_THREADS);
+        cfg.dynamicSmemBytes = LS_TABLE_BYTES;
+        cfg.stream = stream;
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = blocks;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+    }
+    GangLaunch(const GangLaunch&) = delete;
+};
+
+// Blocks for a cluster of `want` (8 or 16): want, 8 where the device places no
+// 16 (a partition with fewer free SMs in a GPC), 0 where it places neither:
+// the general path has to run (a sweep of it takes 140-170 us at any size;
+// local moves take up to half as long again with 8 blocks, two to four times
+// as long with 4).  The device is asked once per kernel.
+template <class A>
+inline int gang_blocks(Context& ctx, void (*kern)(A), int want) {
     static std::mutex mu;
-    static std::map<std::pair<const void*, int>, bool> done;
-    std::lock_guard<std::mutex> lk(mu);
-    bool& d = done[std::make_pair((const void*)kernel, device)];
-    if (d) return;
-    PGGC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    d = true;
+    static std::map<std::pair<const void*, int>, int> largest;
+    if (want == 0) return 0;
+    int most;
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        const auto key = std::make_pair((const void*)kern, ctx.device);
+        auto it = largest.find(key);
+        if (it == largest.end()) {
+            most = 0;
+            if (ctx.max_smem_optin >= LS_TABLE_BYTES) {
+                set_dynamic_smem_once(kern, LS_TABLE_BYTES, ctx.device);
+                PGGC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+                for (int b = 16; b >= 8 && most == 0; b >>= 1) {
+                    GangLaunch g(b, ctx.stream);
+                    int clusters = 0;
+                    if (cudaOccupancyMaxActiveClusters(&clusters, kern, &g.cfg) != cudaSuccess) cudaGetLastError();
+                    else if (clusters > 0) most = b;
+                }
+            }
+            it = largest.emplace(key, most).first;
+        }
+        most = std::min(it->second, ctx.max_cluster);
+    }
+    return most >= want ? want : most >= 8 ? 8 : 0;
 }
 
-// Launches `kern` as one cluster of `blocks` blocks.
+// Launches `kern` as one cluster of `blocks` blocks (from gang_blocks).
 template <class A>
 inline void launch_gang(Context& ctx, void (*kern)(A), const A& a, int blocks) {
-    set_dynamic_smem_once(kern, LS_TABLE_BYTES, ctx.device);
-    set_wide_clusters_once(kern, ctx.device);
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(LS_THREADS);
-    cfg.dynamicSmemBytes = LS_TABLE_BYTES;
-    cfg.stream = ctx.stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = blocks;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    PGGC_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
+    GangLaunch g(blocks, ctx.stream);
+    PGGC_CUDA(cudaLaunchKernelEx(&g.cfg, kern, a));
     PGGC_LAUNCH_CHECK();
 }
 

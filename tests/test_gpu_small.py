@@ -194,3 +194,34 @@ def test_runs(mem, form, weights, method):
     with general_path(mem):
         want = run()
     assert np.array_equal(got[0], want[0]) and got[1] == want[1]
+
+
+@pytest.mark.parametrize("blocks", [15, 8, 7, 0])
+@pytest.mark.parametrize("form", ["one_vertex", "classes_0_to_3", "rows_128_block_tables", "largest_move"])
+def test_device_that_places_no_large_cluster(mem, form, blocks):
+    """Clusters of 8 where 16 cannot be placed, the general path below: the same answers from every step."""
+    hg = _host_graph(form, "float")
+    g = _wgraph(mem, hg, "float")
+
+    def steps():
+        rfd = pg.get_objective(mem, g, pg.OBJ_WMOD)
+        part = np.arange(g.n, dtype=np.int32)
+        l0 = _lib.lib().pggc_launch_count()
+        pg.local_move(mem, g, part, rfd, True)
+        launches = _lib.lib().pggc_launch_count() - l0
+        vcmap, nc = pg.coarsen_leidenR(mem, g, part, rfd, 11, 5)
+        first = part.copy()
+        pg.local_move_strict(mem, g, part, rfd, False)
+        coarse = pg.build_coarse_graph(mem, g, vcmap, nc).to_host()
+        return launches, [first, part, vcmap, nc, rfd.obj, rfd.total_deg(), *coarse]
+
+    steps()  # the products kept with the graph
+    one_launch, want = steps()
+    _lib.check(_lib.lib().pggc_debug_set_cluster_limit(mem.handle, blocks))
+    try:
+        launches, got = steps()
+    finally:
+        _lib.check(_lib.lib().pggc_debug_set_cluster_limit(mem.handle, 16))
+    assert (launches > one_launch) == (blocks < 8)
+    for x, y in zip(got, want):
+        np.testing.assert_array_equal(x, y)
