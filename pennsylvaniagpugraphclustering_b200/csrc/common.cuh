@@ -216,6 +216,14 @@ __host__ __device__ __forceinline__ u32 next_pow2_u32(u32 x) {
     return x + 1;
 }
 
+// Slots of a global hash table for up to `keys` distinct keys: twice that to
+// the next power of two, at most 2^30 (a power above 2^31 leaves 32 bits, and
+// the mask of 0 slots would be the whole address space).
+__host__ __device__ __forceinline__ i64 global_table_slots(i64 keys) {
+    const i64 want = 2 * (keys > 16 ? keys : 16), most = (i64)1 << 30;
+    return next_pow2_u32((u32)(want < most ? want : most));
+}
+
 __host__ __device__ __forceinline__ i64 ceil_div(i64 a, i64 b) { return (a + b - 1) / b; }
 
 // ---------------------------------------------------------------------------

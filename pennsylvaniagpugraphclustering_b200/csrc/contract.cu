@@ -1189,7 +1189,7 @@ std::unique_ptr<Graph<W>> build_coarse_graph(Context& ctx, const Graph<W>& g, co
             off.clear();
             std::vector<i64> ch;
             for (; r1 < n_long; r1++) {
-                const i64 T = next_pow2_u32((u32)(2 * std::max<i64>(std::min<i64>(len[r1], nc), 16)));
+                const i64 T = global_table_slots(std::min<i64>(len[r1], nc));
                 if (r1 > r0 && slots + T > LONG_SLOTS) break;
                 off.push_back(slots);
                 ch.push_back(chunks);
