@@ -66,10 +66,10 @@ WORKLOAD = ("pLeiden+ until stable (ex_iters=-1), WMod, DC-SBM n=4,194,304, deg 
 TARGET_RATIO = 1.5
 Q_TOLERANCE = 0.001
 DOMINANT_FAMILIES = ("select_warp", "select_block", "select_huge", "afterburner_warp", "own_weights", "contract",
-                     "leiden_refine", "filter")
+                     "leiden_refine", "filter", "step_select", "step_afterburner", "step_own", "local_move_small")
 # sub-phases reported beside the families (not candidates for the roofline line)
 SUB_PHASES = ("contract_prep", "contract_hash", "contract_place", "contract_place_big", "host_alloc", "lm_compact",
-              "lm_roundtrip", "lm_newids", "lm_moves", "lm_copy")
+              "lm_roundtrip", "lm_newids", "lm_moves", "lm_copy", "step_moves", "step_objective", "contract_small")
 
 
 def parse():

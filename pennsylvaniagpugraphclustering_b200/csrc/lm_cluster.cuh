@@ -61,6 +61,7 @@ __global__ void __launch_bounds__(LS_THREADS, 1) k_local_move_small(SmallArgs<W>
     bool have_pvals = a.initial == 0;
     if (have_pvals) {
         if (!a.reuse) {
+            if (a.prof) count_own(a, true, a.prof);
             own_step(a, true, a.pvals);
             gang_sync();
             for (i64 i = t0; i < n; i += nt) a.pv_best[i] = a.pvals[i];
@@ -110,6 +111,10 @@ __global__ void __launch_bounds__(LS_THREADS, 1) k_local_move_small(SmallArgs<W>
                 gang_sync();
             }
             s.initial = have_pvals ? 0 : 1;
+            if (a.prof) {
+                count_select(s, a.cls, n, a.prof);
+                gang_sync();  // the select step writes dest
+            }
             select_step<W, CON>(s, a.cls, a.off, L, smem, wb);
             gang_sync();
             if (a.strict) {
@@ -128,6 +133,7 @@ __global__ void __launch_bounds__(LS_THREADS, 1) k_local_move_small(SmallArgs<W>
                 x = 2;
                 break;
             }
+            if (a.prof) count_afterburner(a, a.prof);
             afterburner_step(a, a.cnt + 2 * k, sh);
             gang_sync();
             const i64 nm = (i64)a.cnt[2 * k];
@@ -135,6 +141,10 @@ __global__ void __launch_bounds__(LS_THREADS, 1) k_local_move_small(SmallArgs<W>
             if ((k > 0 || !a.initial) && a.cnt[2 * k + 1] != 0) L = new_ids_step<W, CON>(a, L, sh);
             moves_step(a, have_pvals, FILT ? a.filt.prev_stamp + k + 1 : 0);
             gang_sync();
+            if (a.prof) {
+                count_own(a, !have_pvals, a.prof);
+                gang_sync();  // the step clears the flags
+            }
             own_step(a, !have_pvals, a.pvals);
             have_pvals = true;
             chunk_sums<V>(L, [&](i64 c) { const V t = a.td[c]; return t * t; }, a.partial + a.sq_at, red,
@@ -250,6 +260,7 @@ bool local_move_small(Context& ctx, const Graph<W>& g, const Ordering& ord, i32*
     a.blk = ctx.ws_get<i64>(LM_BLK, 96);
     a.cnt = ctx.ws_get<unsigned long long>(LM_CNT, 2 * LS_MAX_SWEEPS);
     a.sc = ctx.ws_get<LMScalars<V>>(LM_SC, 1);
+    a.prof = ctx.prof_counter("local_move_small");
     a.err = ctx.d_err;
     a.cap = cap;
     a.label_count = best.label_count;

@@ -51,6 +51,7 @@ struct SmallArgs {
     float pm, inv_load;
     int initial, sa, reuse, sweep_limit, keys32;
     int strict;           // one sweep of the strict variant (see below)
+    unsigned long long* prof;  // algorithmic-byte counter (profiling only)
     FiltArgs<W> filt;          // FILT only; prev_stamp is that of the first sweep
     i32* moved_at;
     i32* csize;
@@ -76,6 +77,15 @@ void step_sums(Context& ctx, const SmallArgs<W>& a);
 // state (at most label_bound labels), before the first the starting total
 template <class W>
 void step_objective(Context& ctx, const SmallArgs<W>& a, bool sweep, i64 label_bound);
+
+// The algorithmic bytes of a step that is about to run, added to *prof (NULL:
+// nothing is done): a count of its own, so that the steps carry none.
+template <class W>
+void step_select_bytes(Context& ctx, const SelArgs<W>& s, const i32* cls, i64 count, unsigned long long* prof);
+template <class W>
+void step_afterburner_bytes(Context& ctx, const SmallArgs<W>& a, unsigned long long* prof);
+template <class W>
+void step_own_bytes(Context& ctx, const SmallArgs<W>& a, bool all, unsigned long long* prof);
 
 // Blocks of the cluster that should run a step of this graph, 0 when it is not small.
 int small_cluster_blocks(i64 n, i64 nnz);

@@ -149,6 +149,38 @@ void step_objective(Context& ctx, const SmallArgs<W>& a, bool sweep, i64 label_b
         a, sweep);
     PGGC_LAUNCH_CHECK();
 }
+template <class W>
+__global__ void __launch_bounds__(LS_THREADS) k_step_select_bytes(SelArgs<W> s, const i32* cls, i64 count,
+                                                                  unsigned long long* prof) {
+    count_select(s, cls, count, prof);
+}
+template <class W>
+__global__ void __launch_bounds__(LS_THREADS) k_step_afterburner_bytes(SmallArgs<W> a, unsigned long long* prof) {
+    count_afterburner(a, prof);
+}
+template <class W>
+__global__ void __launch_bounds__(LS_THREADS) k_step_own_bytes(SmallArgs<W> a, bool all, unsigned long long* prof) {
+    count_own(a, all, prof);
+}
+template <class W>
+void step_select_bytes(Context& ctx, const SelArgs<W>& s, const i32* cls, i64 count, unsigned long long* prof) {
+    if (!prof) return;
+    k_step_select_bytes<W><<<step_grid(ctx, ceil_div(count, 32)), LS_THREADS, 0, ctx.stream>>>(s, cls, count, prof);
+    PGGC_LAUNCH_CHECK();
+}
+template <class W>
+void step_afterburner_bytes(Context& ctx, const SmallArgs<W>& a, unsigned long long* prof) {
+    if (!prof) return;
+    k_step_afterburner_bytes<W><<<step_grid(ctx, ceil_div(a.g.n, 32)), LS_THREADS, 0, ctx.stream>>>(a, prof);
+    PGGC_LAUNCH_CHECK();
+}
+template <class W>
+void step_own_bytes(Context& ctx, const SmallArgs<W>& a, bool all, unsigned long long* prof) {
+    if (!prof) return;
+    k_step_own_bytes<W><<<step_grid(ctx, ceil_div(a.g.n, 32)), LS_THREADS, 0, ctx.stream>>>(a, all, prof);
+    PGGC_LAUNCH_CHECK();
+}
+
 #define PGGC_INST_STEP(W)                                                                                \
     template void step_init<W>(Context&, const SmallArgs<W>&);                                           \
     template void step_select<W>(Context&, const SelArgs<W>&, const i32*, const i64*, i64, bool);        \
@@ -156,6 +188,9 @@ void step_objective(Context& ctx, const SmallArgs<W>& a, bool sweep, i64 label_b
     template void step_moves<W>(Context&, const SmallArgs<W>&, bool, i32);                               \
     template void step_own<W>(Context&, const SmallArgs<W>&, bool);                                      \
     template void step_sums<W>(Context&, const SmallArgs<W>&);                                           \
+    template void step_select_bytes<W>(Context&, const SelArgs<W>&, const i32*, i64, unsigned long long*); \
+    template void step_afterburner_bytes<W>(Context&, const SmallArgs<W>&, unsigned long long*);         \
+    template void step_own_bytes<W>(Context&, const SmallArgs<W>&, bool, unsigned long long*);           \
     template void step_objective<W>(Context&, const SmallArgs<W>&, bool, i64);
 PGGC_INST_STEP(i32)
 PGGC_INST_STEP(float)

@@ -481,4 +481,37 @@ __device__ __forceinline__ void filter_step(FiltArgs<W> f, unsigned char* smem) 
     __syncwarp();
 }
 
+// ---- algorithmic bytes (profiling only) ----------------------------------------
+// Counted before a step from the state that it will read, as the class kernels
+// count while they run.
+template <class F>
+__device__ __forceinline__ void count_bytes(i64 k, F f, unsigned long long* prof) {
+    unsigned long long pb = 0;
+    for (i64 x = (i64)blockIdx.x * LS_THREADS + threadIdx.x; x < k; x += (i64)gridDim.x * LS_THREADS) pb += f(x);
+    pb = (unsigned long long)warp_sum_i64((i64)pb);
+    if (lane_id() == 0 && pb) atomicAdd(prof, pb);
+}
+template <class W>
+__device__ __forceinline__ void count_select(const SelArgs<W>& s, const i32* list, i64 count, unsigned long long* prof) {
+    count_bytes(count, [&](i64 x) {
+        const i32 i = list[x];
+        if (s.dest[i] == NO_MOVE) return sel_bytes(s, 0, false);
+        return sel_bytes(s, sel_no_candidate(s, i, sel_prologue(s, i)) ? 0 : s.g.rowptr[i + 1] - s.g.rowptr[i], true);
+    }, prof);
+}
+template <class W>
+__device__ __forceinline__ void count_afterburner(const SmallArgs<W>& a, unsigned long long* prof) {
+    ABArgs<W> ab{};
+    ab.g = a.g;
+    count_bytes(a.g.n, [&](i64 i) {
+        return a.dest[i] == NO_MOVE ? 0ull : ab_bytes(ab, a.g.rowptr[i + 1] - a.g.rowptr[i]);
+    }, prof);
+}
+template <class W>
+__device__ __forceinline__ void count_own(const SmallArgs<W>& a, bool all, unsigned long long* prof) {
+    count_bytes(a.g.n, [&](i64 i) {
+        return all || a.flags[i] ? own_bytes(a.g, a.g.rowptr[i + 1] - a.g.rowptr[i]) : 0ull;
+    }, prof);
+}
+
 }  // namespace pggc

@@ -545,8 +545,7 @@ __global__ void __launch_bounds__(256) k_own_grp(DGraph<W> g, const i32* lab, ty
             } else if (mode == 2) {
                 dest[i] = NULL_PART;
             }
-            // list entry, offsets, own label, result; per edge column, weight, label
-            pb += 4 + 16 + 4 + sizeof(V) + (unsigned long long)(e - b) * (8 + (g.w ? sizeof(W) : 0));
+            pb += own_bytes(g, e - b);
         }
     }
     if (prof) {
@@ -617,7 +616,7 @@ __global__ void __launch_bounds__(256) k_own_small(DGraph<W> g, const i32* lab, 
                     dest[iv[u]] = NULL_PART;
                     flags[iv[u]] = 0;
                 }
-                pb += 4 + 16 + 4 + sizeof(V) + (unsigned long long)(e[u] - b[u]) * (8 + (g.w ? sizeof(W) : 0));
+                pb += own_bytes(g, e[u] - b[u]);
             }
         }
     }
@@ -661,7 +660,7 @@ __global__ void __launch_bounds__(256) k_own_thr(DGraph<W> g, const i32* lab, ty
             dest[i] = NULL_PART;
             flags[i] = 0;
         }
-        pb += 4 + 16 + 4 + sizeof(V) + (unsigned long long)(e - b) * (8 + (g.w ? sizeof(W) : 0));
+        pb += own_bytes(g, e - b);
     }
     if (prof) {
         pb = (unsigned long long)warp_sum_i64((i64)pb);
@@ -1677,6 +1676,7 @@ struct Mover {
         const int tcls = tp.thread_max_deg >= 32 ? 3 : tp.thread_max_deg >= 16 ? 2 : tp.thread_max_deg >= 8 ? 1 : 0;
         const int wend = tp.warp_max_deg >= 127 ? 4 : 3;  // first class after the warp kernel's
         if (ord.off_large > 0 && steps) {
+            step_select_bytes<W>(ctx, a, cls.list, ord.off_large, ctx.prof_counter("step_select"));
             ProfScope ps(ctx, "step_select");
             step_select<W>(ctx, a, cls.list, cls.off, ord.off_large, CON);
         } else if (ord.off_large > 0) {
@@ -1948,9 +1948,16 @@ struct Mover {
         update_objective_dev(lambda, label_bound);
     }
 
+    void own_step(bool all) {
+        step_own_bytes<W>(ctx, sa, all, ctx.prof_counter("step_own"));
+        ProfScope ps(ctx, "step_own");
+        step_own<W>(ctx, sa, all);
+    }
+
     // The rest of a sweep after its select, a launch per step.  False: nothing
     // moves and the sweep's loop ends.
     bool step_sweep(i64& label_bound, bool may_append, i32* constraint, i64* total_moves) {
+        step_afterburner_bytes<W>(ctx, sa, ctx.prof_counter("step_afterburner"));
         {
             ProfScope ps(ctx, "step_afterburner");
             step_afterburner<W>(ctx, sa);
@@ -1970,10 +1977,13 @@ struct Mover {
             set_new_cluster_ids(nm, constraint);
             label_bound = std::min<i64>(label_bound + n_new, cap);
         }
-        ProfScope pm(ctx, "step_moves");
-        step_moves<W>(ctx, sa, cdata_init, ctx.filt.stamp);
-        step_own<W>(ctx, sa, !cdata_init);
+        {
+            ProfScope pm(ctx, "step_moves");
+            step_moves<W>(ctx, sa, cdata_init, ctx.filt.stamp);
+        }
+        own_step(!cdata_init);
         cdata_init = true;
+        ProfScope po(ctx, "step_objective");
         step_sums<W>(ctx, sa);
         step_objective<W>(ctx, sa, true, label_bound);
         *total_moves += nm;
@@ -2147,7 +2157,7 @@ void local_move(Context& ctx, const Graph<W>& g, const Ordering& ord, i32* best_
         m.step_args(best, best_part, best.total_deg.p, is_initial, reuse);
         m.cdata_init = !is_initial;
         if (!is_initial) {
-            if (!reuse) step_own<W>(ctx, m.sa, true);
+            if (!reuse) m.own_step(true);
             step_sums<W>(ctx, m.sa);
             step_objective<W>(ctx, m.sa, false, 0);
         }

@@ -361,6 +361,13 @@ __device__ __forceinline__ unsigned long long ab_bytes(const ABArgs<W>& a, i64 d
     return 41ull + (unsigned long long)deg * (8ull + wb);
 }
 
+// algorithmic bytes of one own-cluster weight: list entry, offsets, own label,
+// result; per edge column, weight, label
+template <class W>
+__device__ __forceinline__ unsigned long long own_bytes(const DGraph<W>& g, i64 deg) {
+    return 24ull + sizeof(typename Traits<W>::V) + (unsigned long long)deg * (8 + (g.w ? sizeof(W) : 0));
+}
+
 // Rows are summed G lanes at a time, UG groups of edges in flight: the columns
 // of all of them are loaded, then their first gathers, then what those ask
 // for.  One edge after another, a row of 2,000 edges was a chain of 63 times

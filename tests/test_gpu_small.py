@@ -225,3 +225,40 @@ def test_device_that_places_no_large_cluster(mem, form, blocks):
     assert (launches > one_launch) == (blocks < 8)
     for x, y in zip(got, want):
         np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("strict", [False, True])
+@pytest.mark.parametrize("form,weights", [("one_vertex", None), ("classes_0_to_3", "float"), ("largest_move", None),
+                                          ("steps_40k", "float"), ("steps_40k", None), ("steps_hubs", "int")])
+def test_profile_counts_the_same_bytes(mem, form, weights, strict):
+    """The algorithmic bytes of a local move do not depend on the path that runs it."""
+    hg = _host_graph(form, weights)
+    g = _wgraph(mem, hg, weights)
+    ct = _lib.ctypes
+
+    def counted():
+        rfd = pg.get_objective(mem, g, _objective(weights))
+        part = np.arange(g.n, dtype=np.int32)
+        pg.local_move(mem, g, part, rfd, True, sweep_limit=-1 if strict else 2)
+        _lib.check(_lib.lib().pggc_profile_reset(mem.handle))
+        _lib.check(_lib.lib().pggc_profile_enable(mem.handle, 1))
+        try:
+            (pg.local_move_strict if strict else pg.local_move)(mem, g, part, rfd, False)
+        finally:
+            _lib.check(_lib.lib().pggc_profile_enable(mem.handle, 0))
+        out = {}
+        for f in ("select_warp", "select_block", "select_huge", "afterburner_warp", "own_weights", "step_select",
+                  "step_afterburner", "step_own", "local_move_small"):
+            launches, ms, nbytes = ct.c_int64(), ct.c_double(), ct.c_double()
+            _lib.check(_lib.lib().pggc_profile_read(mem.handle, f.encode(), ct.byref(launches), ct.byref(ms),
+                                                    ct.byref(nbytes)))
+            out[f] = (launches.value, nbytes.value)
+        return out
+
+    got = counted()
+    with general_path(mem):
+        want = counted()
+    if strict and got["select_warp"][0]:
+        return  # candidates: the one-launch sweep came before the general path's
+    assert got["select_warp"][0] == 0 and want["local_move_small"][0] == want["step_select"][0] == 0
+    assert sum(b for _, b in got.values()) == sum(b for _, b in want.values()) > 0
