@@ -255,16 +255,29 @@ def test_trained_filter_skips_work_at_equal_modularity(mem):
     assert learned["objective"] >= plain["objective"] - 0.001
 
 
-@pytest.mark.parametrize("n", [127, 128, 129, 128 * 296, 128 * 296 + 1])
-def test_mlp_loss_grad_tile_edges(mem, n):
-    """Batches that end inside, at and past a 128-sample tile and the blocks' first round of tiles."""
+@pytest.mark.parametrize("tiles,extra", [(1, -1), (1, 0), (1, 1), (None, 0), (None, 1)])
+def test_mlp_loss_grad_tile_edges(mem, tiles, extra):
+    """Batches that end inside, at and past a 128-sample tile and the blocks' first round of tiles (None).  The samples
+    at the edges have large features and the wrong label: without one of them, or with one twice, the gradient is off
+    by far more than the tolerance (checked on the oracle)."""
+    if tiles is None:
+        torch = pytest.importorskip("torch")
+        tiles = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    n = 128 * tiles + extra
     p = M.init_params(21)
     p[M.O_B1:M.O_W2] = 0.05
     x = _features(n, 22)
+    edges = [e for e in {0, 127, 128, n - 2, n - 1} if 0 <= e < n]
+    x[edges] *= np.float32(n / 16)
     y = _teacher_labels(x, 23)
+    y[edges] = (M.forward(p, x[edges])[0] < 0).astype(np.float32)
     loss, g = MF.loss_grad(mem, p, x, y, 2.0)
     loss_o, g_o = M.loss_and_grad(p, x, y, 2.0)
     # FP32 chains of 128 samples and a few hundred tile sums: about (128 + 300) 2^-24 of the sum of magnitudes,
     # and single activations that round to the other BF16 neighbour
-    assert abs(loss - loss_o) <= 1e-5 * (1.0 + abs(loss_o))
-    assert np.abs(g - g_o).max() <= 1e-3 * np.abs(g_o).max() + 1e-7
+    tol_loss, tol_g = 1e-5 * (1.0 + abs(loss_o)), 1e-3 * np.abs(g_o).max() + 1e-7
+    for e in edges:
+        loss_e, g_e = M.loss_and_grad(p, x[e:e + 1], y[e:e + 1], 2.0)
+        assert abs(loss_e) / n > 20 * tol_loss and np.abs(g_e).max() / n > 20 * tol_g
+    assert abs(loss - loss_o) <= tol_loss
+    assert np.abs(g - g_o).max() <= tol_g

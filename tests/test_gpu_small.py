@@ -11,7 +11,9 @@ import numpy as np
 import pytest
 
 import pennsylvaniagpugraphclustering_b200 as pg
+from oracle import mlp_oracle as M
 from pennsylvaniagpugraphclustering_b200 import _lib
+from pennsylvaniagpugraphclustering_b200 import move_filter as MF
 from pennsylvaniagpugraphclustering_b200.graphgen import HostGraph
 
 pytestmark = pytest.mark.gpu
@@ -262,3 +264,57 @@ def test_profile_counts_the_same_bytes(mem, form, weights, strict):
         return  # candidates: the one-launch sweep came before the general path's
     assert got["select_warp"][0] == 0 and want["local_move_small"][0] == want["step_select"][0] == 0
     assert sum(b for _, b in got.values()) == sum(b for _, b in want.values()) > 0
+
+
+def _one_feature(f, sign):
+    """A network whose logit is sign * feature f."""
+    p = np.zeros(M.N_PARAMS, np.float32)
+    p[M.O_W1 + f], p[M.O_W1 + 8 + f] = sign, -sign
+    p[M.O_W2], p[M.O_W2 + 32 + 1] = 1, 1
+    p[M.O_W3], p[M.O_W3 + 1] = 1, -1
+    return p
+
+
+# networks that reject some vertices: by the share of weight inside, the last gain, having moved in the last sweep,
+# the size and the volume of the cluster, the sweep's number, and by all features at once
+NETS = {"inside": (_one_feature(1, -1), -0.6), "gain": (_one_feature(2, -1), -0.1), "moved": (_one_feature(3, -1), -0.5),
+        "size": (_one_feature(4, -1), -0.2), "volume": (_one_feature(5, -1), None), "sweep": (_one_feature(7, -1), -0.3),
+        "all": (M.init_params(3), 0.05)}
+
+
+@pytest.mark.parametrize("net", list(NETS))
+@pytest.mark.parametrize("form,weights", [("classes_0_to_3", "float"), ("largest_move", None), ("steps_40k", "float"),
+                                          ("steps_hubs", None)])
+def test_filtered_moves(mem, form, weights, net):
+    """The filter's features and counts are those of the class kernels: the same vertices are skipped."""
+    hg = _host_graph(form, weights)
+    g = _wgraph(mem, hg, weights)
+    params, threshold = NETS[net]
+    if threshold is None:
+        threshold = -6.0 / g.n  # six vertices' share of the volume
+
+    def run():
+        MF.enable(mem, params, threshold)
+        MF.stats(mem, reset=True)
+        try:
+            rfd = pg.get_objective(mem, g, _objective(weights))
+            part = np.arange(g.n, dtype=np.int32)
+            out = []
+            for initial in (True, False):
+                st = pg.local_move(mem, g, part, rfd, initial)
+                out.append((part.copy(), st["sweeps"], st["moves"], rfd.obj, *MF.stats(mem)))
+            rfd = pg.get_objective(mem, g, _objective(weights))
+            labels, st = pg.run_clustering(mem, g, rfd, method=pg.METHOD_LEIDEN_PLUS, ex_iters=0, seed=9)
+            out.append((labels, *st.values(), *MF.stats(mem)))
+        finally:
+            MF.disable(mem)
+        return out
+
+    got = run()
+    with general_path(mem):
+        want = run()
+    for a, b in zip(got, want):
+        for x, y in zip(a, b):
+            np.testing.assert_array_equal(x, y)
+    evaluated, skipped = got[1][-2:]
+    assert evaluated > 0 and skipped > 0
