@@ -9,13 +9,20 @@ namespace pggc {
 // Above these a launch per step over the whole GPU is the faster way: the work
 // on the cluster's 16 SMs grows with the edges while the launches do not.
 // Local moves have the lower limits (their steps cover the GPU in 7 launches a
-// sweep, contraction and refinement take 25 to 30): six sweeps over 57 K edges
-// take 356 us either way, over 227 K edges of 14 a row 687 us here and 465 us
-// there; over 143 K edges of 143 a row 384 and 490 us, over 175 K 507 and 570.
+// sweep, contraction and refinement take 25 to 30), on the edges plus what a
+// vertex costs beside its edges, about four of them.  Six sweeps here and with
+// a launch per step, us (planted partitions / power-law degrees):
+//   mean degree 4:    49 K edges 371, 421 / 496, 499; 127 K 667, 468 / 938, 520
+//   mean degree 8:    68 K edges 377, 412 / 511, 516; 155 K 559, 455 / 941, 532
+//   mean degree 15:   57 K edges 329, 441; 104 K 447, 444 / 598, 599; 227 K 704, 464
+//   mean degree 30:   81 K edges 370, 459 / 497, 603; 144 K 531, 469 / 805, 691
+// Long rows go further, a warp or block has enough to do in each:
+//   mean degree 55:  133 K edges 459, 451;  75: 158 K 362, 386 (FP32 weights 520,
+//   512);  94: 170 K 311, 369 (446, 490);  136: 130 K 189, 307 (335, 472)
 constexpr i64 LS_MAX_N = 32768;
 constexpr i64 LS_MAX_NNZ = 262144;
-constexpr i64 LS_MOVE_NNZ = 131072;
-constexpr i64 LS_MOVE_NNZ_LONG = 196608;  // mean degree of 64 or more
+constexpr i64 LS_MOVE_SIZE = 114688;      // edges plus four a vertex
+constexpr i64 LS_MOVE_NNZ_LONG = 196608;  // edges, at a mean degree of 64 or more
 constexpr i64 LS_MAX_LABELS = 131072;
 
 constexpr int LS_MAX_SWEEPS = 6;
@@ -128,9 +135,10 @@ struct GangLaunch {
 
 // Blocks for a cluster of `want` (8 or 16): want, 8 where the device places no
 // 16 (a partition with fewer free SMs in a GPC), 0 where it places neither:
-// the general path has to run (a sweep of it takes 140-170 us at any size;
-// local moves take up to half as long again with 8 blocks, two to four times
-// as long with 4).  The device is asked once per kernel.
+// the general path has to run (local moves take up to half as long again with
+// 8 blocks as with 16 and up to 2.4 times as long with 4, see
+// small_cluster_blocks; the launches of the general path 1.3 to 2 times).  The
+// device is asked once per kernel.
 template <class A>
 inline int gang_blocks(Context& ctx, void (*kern)(A), int want) {
     static std::mutex mu;

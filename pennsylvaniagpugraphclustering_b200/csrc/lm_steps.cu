@@ -195,12 +195,11 @@ void step_own_bytes(Context& ctx, const SmallArgs<W>& a, bool all, unsigned long
 PGGC_INST_STEP(i32)
 PGGC_INST_STEP(float)
 
-// Sixteen blocks (the largest cluster) were the fastest from 1,000 vertices up:
-// six sweeps of a 1,000-vertex SBM (14 K edges) take 551 / 390 / 303 / 266 us
-// with 1 / 4 / 8 / 16 blocks, of a 16,000-vertex one (227 K edges) 7.95 / 2.36
-// / 1.33 / 0.92 ms (lane groups in every class), and a batch of 48
-// graphs on 16 streams 60 / 46 / 40 ms with 4 / 8 / 16; at 300 vertices 8 and
-// 16 blocks are equal.
+// Sixteen blocks (the largest cluster) are the fastest from 1,000 vertices up:
+// six sweeps of an SBM of mean degree 14 take 456 / 293 / 239 / 205 us with 1 /
+// 4 / 8 / 16 blocks at 1,000 vertices, 1,627 / 618 / 421 / 333 us at 4,000, and
+// 2,096 / 682 / 429 / 320 us at 1,000 vertices of 83 FP32 edges; at 300
+// vertices (4 K edges) 232 / 205 / 168 / 167.
 int small_cluster_blocks(i64 n, i64 nnz) {
     if (n > LS_MAX_N || nnz > LS_MAX_NNZ) return 0;
     return nnz + 4 * n <= 4096 ? 8 : 16;

@@ -201,8 +201,10 @@ __device__ __forceinline__ i64 select_low(const SelArgs<W>& a, const i32* cls, c
     // A thread per vertex from about six (degree 17-32) to twelve (up to 8)
     // vertices a warp: a lane group issues 150 instructions a vertex of the
     // 17-32 class, a thread a third of that, but its chain is longer.  Select
-    // step of a 65,536-vertex graph: 31.7 us with groups, 26.7 us so; local
-    // move of a 16,000-vertex one 0.91 -> 0.72 ms.
+    // step of a 65,536-vertex graph: 31.7 us with groups, 26.7 us so.  One-
+    // launch local moves, us with groups / so: 6,000 vertices of 14 edges 472 /
+    // 409 (FP32 521 / 473), 8,000 of 8 edges 401 / 314; with a launch per
+    // step, 65,536 vertices of 14 edges 626 / 594.
     auto thr = [&](auto kc, i64 lo, i64 hi) {
         constexpr int K = decltype(kc)::value;
         const i64 first = gang_first(rot);

@@ -2104,8 +2104,16 @@ struct Mover {
 };
 
 // One launch per step and all degree classes: graphs whose per-class kernels
-// are too short for their launches.  Logging, rows summed by 1024 threads,
-// tuned degree bounds and injected probe faults keep the class kernels.
+// are too short for their launches.  The steps pass over all vertices where the
+// class kernels compact the few that moved, so they lose with size where little
+// moves.  A first local move and a second from its result, ms with steps /
+// with class kernels (power-law degrees, 20 edges a row, FP32):
+//   0.5 M vertices 3.09 / 4.03, 2.09 / 2.71;  1 M 5.64 / 6.63, 3.35 / 3.69
+//   2 M 10.6 / 11.6, 6.31 / 6.22;  4.2 M 21.9 / 22.4, 11.6 / 10.4
+// (planted partition, 14 edges a row, unit weights: 1 M 2.53 / 3.06, 2.07 /
+// 2.26; 2 M 4.94 / 5.29, 3.64 / 3.55).
+// Logging, rows summed by 1024 threads, tuned degree bounds and injected probe
+// faults keep the class kernels.
 constexpr i64 STEP_MAX_N = (i64)1 << 20;
 template <class W>
 static bool step_path(const Context& ctx, const Graph<W>& g, const Ordering& ord, i64 label_count) {

@@ -69,7 +69,8 @@ FORMS = {
     "rows_128_warp_tables": (700, 350, 200, 40, 0, 0),       # labels fit a warp's share
     "rows_128_block_tables": (3000, 60, 10, 4, 40, 400),      # they do not
     "rows_4096": (30000, 60, 2, 1, 3, 5500),                  # several passes of the table
-    "largest_move": (32768, 128, 2, 1.5, 0, 0),               # one launch for every step
+    "largest_move": (32768, 128, 2, 1.5, 0, 0),               # the most vertices, few edges
+    "move_16k": (16000, 128, 2, 1, 0, 0),                     # close to the one-launch move's limit
     "largest": (32768, 128, 5, 2, 0, 0),                      # one launch for contraction and refinement
     "steps_40k": (40000, 100, 9, 3, 30, 400),                 # a launch per step
     "steps_hubs": (50000, 60, 6, 2, 3, 6000),
@@ -181,6 +182,7 @@ def test_contraction(mem, form, nc, weights):
 @pytest.mark.parametrize("method", [pg.METHOD_LOUVAIN, pg.METHOD_LEIDEN, pg.METHOD_LEIDEN_PLUS])
 @pytest.mark.parametrize("form,weights", [("chunk_edge", None), ("classes_0_to_3", "float"),
                                           ("rows_128_block_tables", "int"), ("largest_move", "float"), ("largest", "float"),
+                                          ("move_16k", "int"),
                                           ("steps_40k", "float"), ("steps_hubs", "int")])
 def test_runs(mem, form, weights, method):
     hg = _host_graph(form, weights)
@@ -199,7 +201,7 @@ def test_runs(mem, form, weights, method):
 
 
 @pytest.mark.parametrize("blocks", [15, 8, 7, 0])
-@pytest.mark.parametrize("form", ["one_vertex", "classes_0_to_3", "rows_128_block_tables", "largest_move"])
+@pytest.mark.parametrize("form", ["one_vertex", "classes_0_to_3", "rows_128_block_tables", "move_16k"])
 def test_device_that_places_no_large_cluster(mem, form, blocks):
     """Clusters of 8 where 16 cannot be placed, the general path below: the same answers from every step."""
     hg = _host_graph(form, "float")
@@ -230,7 +232,7 @@ def test_device_that_places_no_large_cluster(mem, form, blocks):
 
 
 @pytest.mark.parametrize("strict", [False, True])
-@pytest.mark.parametrize("form,weights", [("one_vertex", None), ("classes_0_to_3", "float"), ("largest_move", None),
+@pytest.mark.parametrize("form,weights", [("one_vertex", None), ("classes_0_to_3", "float"), ("move_16k", None),
                                           ("steps_40k", "float"), ("steps_40k", None), ("steps_hubs", "int")])
 def test_profile_counts_the_same_bytes(mem, form, weights, strict):
     """The algorithmic bytes of a local move do not depend on the path that runs it."""
@@ -283,7 +285,7 @@ NETS = {"inside": (_one_feature(1, -1), -0.6), "gain": (_one_feature(2, -1), -0.
 
 
 @pytest.mark.parametrize("net", list(NETS))
-@pytest.mark.parametrize("form,weights", [("classes_0_to_3", "float"), ("largest_move", None), ("steps_40k", "float"),
+@pytest.mark.parametrize("form,weights", [("classes_0_to_3", "float"), ("move_16k", None), ("steps_40k", "float"),
                                           ("steps_hubs", None)])
 def test_filtered_moves(mem, form, weights, net):
     """The filter's features and counts are those of the class kernels: the same vertices are skipped."""
@@ -318,3 +320,28 @@ def test_filtered_moves(mem, form, weights, net):
             np.testing.assert_array_equal(x, y)
     evaluated, skipped = got[1][-2:]
     assert evaluated > 0 and skipped > 0
+
+
+@pytest.mark.parametrize("n,d,fits", [(8192, 10, True), (8193, 10, False),    # edges plus four a vertex: 114,688
+                                      (1737, 62, True), (1738, 62, False),
+                                      (3072, 64, True), (3073, 64, False)])   # long rows: 196,608 edges
+def test_size_limits_of_the_one_launch_move(mem, n, d, fits):
+    """Rings where every vertex has d neighbours, at the limits and just above: the path that runs, and its answer."""
+    col = np.sort((np.arange(n)[:, None] + np.delete(np.arange(-(d // 2), d // 2 + 1), d // 2)) % n, axis=1)
+    g = pg.weighted_graph(mem, np.arange(n + 1, dtype=np.int64) * d, col.astype(np.int32).ravel(), None,
+                          objective=pg.OBJ_MOD)
+
+    def move():
+        rfd = pg.get_objective(mem, g, pg.OBJ_MOD)
+        part = np.arange(n, dtype=np.int32)
+        l0 = _lib.lib().pggc_launch_count()
+        st = pg.local_move(mem, g, part, rfd, True)
+        return _lib.lib().pggc_launch_count() - l0, (part, st["sweeps"], st["moves"], rfd.obj)
+
+    move()  # the products kept with the graph
+    launches, got = move()
+    assert (launches <= 3) == fits  # label check and move
+    with general_path(mem):
+        _, want = move()
+    for x, y in zip(got, want):
+        np.testing.assert_array_equal(x, y)
