@@ -315,9 +315,9 @@ __global__ void __launch_bounds__(CW_WARPS * 32) k_contract_warp(CArgs<W> a, con
 }
 
 // block per coarse row; the table is in shared memory (`gcap` slots, sized to
-// the bucket's largest table) or, with GLOBAL, in a per-block global region.
-// With OVF (shared tables of gcap slots smaller than 2U), a row whose distinct
-// keys do not fit is appended to `ovf_list` for the global-table pass instead.
+// the bucket's largest table).  With OVF (tables of gcap slots smaller than
+// 2U), a row whose distinct keys do not fit is appended to `ovf_list`, the
+// list of long rows (k_long_insert, k_long_write), instead.
 template <class W, int THREADS = 256, bool OVF = false>
 __global__ void __launch_bounds__(THREADS) k_contract_block(CArgs<W> a, const i32* list, const i64* d_count, i64 gcap, i64 nc,
                                                             i32* ovf_list = nullptr, i64* ovf_count = nullptr) {
@@ -934,8 +934,8 @@ __global__ void k_big_place(const i32* list, i64 count, const i64* tstart, const
 // Sorts the coarse rows into the hashing buckets in one pass (list order is
 // irrelevant: rows are independent).  Buckets by bound (sum of member degrees)
 // and U = min(bound, nc): 0: bound <= 32, 1: bound <= 256, 2: U <= 1024,
-// 3: U <= 4096, 4: above.  cnt[k] counts bucket k; cnt[5] is the largest
-// bound of bucket 4.
+// 3: U <= 4096, 4: above; 5: bound > LONG_ROW, whatever U is.  cnt[k] counts
+// bucket k.
 __global__ void k_bucket_rows(const i64* P, const i64* cstart, i64 nc, i32* l0, i32* l1, i32* l2, i32* l3, i32* l4,
                               i32* l5, unsigned long long* cnt) {
     const int l = lane_id();
@@ -1078,7 +1078,7 @@ std::unique_ptr<Graph<W>> build_coarse_graph(Context& ctx, const Graph<W>& g, co
     // min(bound, nc): small warp rows (bound <= 32), medium warp rows
     // (bound <= 256), block rows with shared tables of 2048 slots (U <= 1024)
     // and 8192 slots (U <= 4096), big rows with 16384-slot shared tables
-    // (U > 4096) whose overflow falls back to global tables
+    // (U > 4096) whose overflow joins the long rows
     WsBuf<i32> lw(ctx, CS_LW, nc), lm(ctx, CS_LM, nc), lb(ctx, CS_LB, nc), lb2(ctx, CS_LB2, nc), lh(ctx, CS_LH, nc),
         lo(ctx, CS_LO, nc);
     // counts: [0] small warp rows, [1] medium warp rows, [2] 2048-slot block
@@ -1093,7 +1093,7 @@ std::unique_ptr<Graph<W>> build_coarse_graph(Context& ctx, const Graph<W>& g, co
                                                    (unsigned long long*)counts.p);
         PGGC_LAUNCH_CHECK();
     }
-    // one round trip: bucket sizes and the largest big-row bound
+    // one round trip: bucket sizes
     const i64* hc = (const i64*)ctx.readback(counts.p, 16 * sizeof(i64));
     const i64 n_w = hc[0], n_m = hc[1], n_b = hc[2], n_b2 = hc[3], n_h = hc[4];
     i64 n_long = hc[5];

@@ -161,10 +161,6 @@ __device__ __forceinline__ void row_block(const CSmallArgs<W>& a, i32 c, unsigne
     if (threadIdx.x == 0) a.ucount[c] = (i32)(at - first);
 }
 
-__device__ __forceinline__ int small_deg_class(i32 d) {
-    return d <= 8 ? 0 : d <= 16 ? 1 : d <= 32 ? 2 : d < LARGE_CUTOFF ? 3 : d <= 1024 ? 4 : d <= HUGE_DEG ? 5 : 6;
-}
-
 template <class W>
 __global__ void __launch_bounds__(LS_THREADS, 1) k_contract_small(CSmallArgs<W> a) {
     using V = typename Traits<W>::V;
@@ -278,7 +274,7 @@ __global__ void __launch_bounds__(LS_THREADS, 1) k_contract_small(CSmallArgs<W> 
         for (i64 x0 = lo; x0 < hi; x0 += LS_THREADS) {
             const i64 x = x0 + threadIdx.x;
             const i32 d = x < hi ? a.ucount[x] : -1;
-            const int k = d >= 0 ? small_deg_class(d) : -1;
+            const int k = d >= 0 ? deg_class(d) : -1;
             sum += d > 0 ? d : 0;
             mx = max(mx, d);
             c0 += __syncthreads_count(d >= 0 && d < LARGE_CUTOFF);
@@ -357,7 +353,7 @@ __global__ void __launch_bounds__(LS_THREADS, 1) k_contract_small(CSmallArgs<W> 
             p0 += a0;
             p1 += a1;
             p2 += min((i64)LS_THREADS, hi - x0) - a0 - a1;
-            const int k = d >= 0 ? small_deg_class(d) : -1;
+            const int k = d >= 0 ? deg_class(d) : -1;
 #pragma unroll
             for (int q = 0; q < NCLS; q++) {
                 const unsigned m = __ballot_sync(FULL, k == q);

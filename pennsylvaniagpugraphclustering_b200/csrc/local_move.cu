@@ -1931,8 +1931,9 @@ struct Mover {
             own_weights_impl<W>(ctx, g, ord, part.p, pvals.p, 1, flags.p, dest.p, &cls);
         } else {
             // few moves with few neighbours and no hubs (flags cost a pass over all
-            // vertices, the list an atomic per neighbour by the mover's warp): list the affected vertices once and recompute only them
-            // (the same per-vertex association as the class kernels)
+            // vertices, the list an atomic per neighbour by the mover's warp): list
+            // the affected vertices once and recompute only them (the same
+            // per-vertex association as the class kernels)
             if (++epoch == 0) {
                 PGGC_CUDA(cudaMemsetAsync(stamp.p, 0, sizeof(u32) * std::max<i64>(n, 1), ctx.stream));
                 epoch = 1;
