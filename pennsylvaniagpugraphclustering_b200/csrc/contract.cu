@@ -249,9 +249,11 @@ __device__ __forceinline__ typename Traits<W>::V cchunk_load(const CArgs<W>& a, 
 // the entry of one lane, for tables in units
 template <class W>
 __device__ __forceinline__ i32 centry(const CArgs<W>& a, i64 q, i64 qend, const Units<W>& un, i64& x) {
-    const i32 key = q < qend ? a.fkey[q] : -1;
-    x = 0;
-    if (key >= 0) x = a.g.w ? un.of(a.fw[q]) : un.of(W(1));
+    const bool in = q < qend;
+    const i32 key = in ? a.fkey[q] : -1;
+    // not asked of the key: the two loads go out together
+    const W wv = in && a.g.w ? a.fw[q] : W(1);
+    x = key >= 0 ? un.of(wv) : 0;
     return key;
 }
 
