@@ -478,14 +478,20 @@ __global__ void __launch_bounds__(THREADS) k_contract_dense(CArgs<W> a, const i3
 
 // ---- long rows, split across blocks -------------------------------------------
 // Rows of more than LONG_ROW member edges, and rows whose distinct keys
-// overflowed the shared table.  A block per row left these to one SM each: a
+// overflowed the shared table.  A block per row leaves these to one SM each: a
 // cluster of R-MAT's core has tens of millions of member edges (19 ms for one
-// contraction), a planted partition's 455 clusters 20,000 each (33 ms).  Each
-// row owns a global table; a block merges LONG_CHUNK edges in a shared table
-// first (keys that do not fit go straight to the global one) and adds its
-// distinct keys to the row's, so the global atomics are few where the keys
-// repeat; then blocks over table slots write the row's entries.
-constexpr i64 LONG_ROW = 16384;
+// contraction).  Each row owns a global table; a block merges LONG_CHUNK edges
+// in a shared table first (keys that do not fit go straight to the global one)
+// and adds its distinct keys to the row's, so the global atomics are few where
+// the keys repeat; then blocks over table slots write the row's entries.
+// The line: a table pass over all slots and the second level of atomics cost
+// more than a block's own pass until the row is the longest work of the launch.
+// Contraction with the line at 16 K / 64 K / 128 K / 1 M member edges, us:
+// 4.2 M-vertex DC-SBM by its local move (41,668 rows, 1,319 above 16 K) 4,748 /
+// 3,431 / 3,051 / 3,056, its level 1 (600 above 16 K) 3,770 / 3,187 / 3,196 /
+// 3,217, 455 clusters of 43 K edges 383 / 316 / 341 / 308, 60 clusters of 332 K
+// edges 1,118 / 1,116 / 1,119 / 1,863.
+constexpr i64 LONG_ROW = 131072;
 constexpr int LONG_CHUNK = 16384;
 constexpr int LONG_THREADS = 512;
 constexpr int LONG_TS = 4096;

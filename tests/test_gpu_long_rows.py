@@ -185,3 +185,40 @@ def test_rows_of_more_edges_than_vertices(mem, how, weights):
             MF.log_stop(mem, 1 << 16)
     assert st["moves"] == k and np.array_equal(part[a], part[a + 1]) and np.array_equal(part[a], part[a + 2])
     assert rfd.get_objective() == pytest.approx(pg.verify_objective(mem, g, part, objective)[0], rel=1e-12)
+
+
+@pytest.mark.parametrize("weights", [None, "int", "float"])
+def test_contraction_at_the_long_row_limit(mem, weights):
+    """Rows of exactly 131,072 member edges (a block's), just above (split across blocks), and of 80,000 with more
+    distinct keys than the largest shared table (handed over by the block)."""
+    d, n = 32, 120000
+    u = np.repeat(np.arange(n), d)
+    v = (u + np.tile(np.concatenate([np.arange(-16, 0), np.arange(1, 17)]) * 1201, n)) % n
+    o = np.lexsort((v, u))
+    src, col = u[o], v[o].astype(np.int32)
+    w = None
+    if weights:
+        k = (np.minimum(src, col).astype(np.int64) * n + np.maximum(src, col)) * 2654435761 % 1000003
+        w = (k % 9 - 2).astype(np.int32) if weights == "int" else ((k + 1) * 2.0 ** -20).astype(np.float32)
+    g = pg.weighted_graph(mem, np.arange(n + 1, dtype=np.int64) * d, col, w,
+                          objective=pg.OBJ_WMOD if weights else pg.OBJ_MOD)
+    nc = 60003
+    m = 3 + np.random.default_rng(1).permutation(np.arange(n) % (nc - 3))
+    m[:4096] = 0
+    m[50000:54097] = 1
+    spread = np.arange(60000, n)[::24][:2500]
+    m[spread] = 2
+    vcmap = np.unique(m, return_inverse=True)[1].astype(np.int32)
+    nc = int(vcmap.max()) + 1
+    assert [d * int((vcmap == c).sum()) for c in range(3)] == [131072, 131104, 80000]
+    crow, ccol, cw, _ = pg.build_coarse_graph(mem, g, vcmap, nc).to_host()
+    a, b = vcmap[src].astype(np.int64), vcmap[col].astype(np.int64)
+    keep = a != b
+    key, inv = np.unique(a[keep] * nc + b[keep], return_inverse=True)
+    assert np.sum(key // nc == 2) > 16384
+    wide = np.float64 if weights == "float" else np.int64
+    total = np.zeros(len(key), wide)
+    np.add.at(total, inv, np.ones(int(keep.sum()), wide) if w is None else w[keep].astype(wide))
+    assert np.array_equal(crow, np.concatenate([[0], np.cumsum(np.bincount(key // nc, minlength=nc))]))
+    assert np.array_equal(ccol, key % nc)
+    assert np.array_equal(cw, total.astype(np.float32 if weights == "float" else np.int32))
