@@ -37,6 +37,12 @@ __device__ __forceinline__ void cvatomic_add(i64* a, i64 x) {
     else ::atomicAdd((unsigned long long*)a, (unsigned long long)x);
 }
 __device__ __forceinline__ void cvatomic_add(double* a, double x) { ::atomicAdd(a, x); }
+// An i64 of a shared table that only counts edges (unit weights, fewer than
+// 2^32 in a row): the low word alone, one atomic without a result.
+struct Count {
+    u32 lo, hi;
+};
+__device__ __forceinline__ void cvatomic_add(Count* a, Count x) { ::atomicAdd(&a->lo, x.lo); }
 
 template <class W>
 __global__ void k_contract_count(DGraph<W> g, const i32* vcmap, i64* cnt, i64* bound) {
@@ -263,7 +269,9 @@ __device__ __forceinline__ void cchunk(const CArgs<W>& a, i64 q, i64 qend, i32* 
     if (un.on) {
         i64 x;
         const i32 k = centry(a, q, qend, un, x);
-        if (k >= 0) ctable_add(keys, (i64*)vals, mask, k, x, a.err, a.probe_cap);
+        if (k < 0) return;
+        if (a.g.w) ctable_add(keys, (i64*)vals, mask, k, x, a.err, a.probe_cap);
+        else ctable_add(keys, (Count*)vals, mask, k, Count{1, 0}, a.err, a.probe_cap);
         return;
     }
     i32 key;
