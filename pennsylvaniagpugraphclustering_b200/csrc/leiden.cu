@@ -544,6 +544,7 @@ struct TsIn<double> {
 // inner connectivity: edges to earlier members of the same tree
 template <class W>
 struct InnerRow {
+    static constexpr int BATCH = UG;
     const DGraph<W>& g;
     const i32 *vcmap, *order;
     i32 c, o;

@@ -222,3 +222,42 @@ def test_contraction_at_the_long_row_limit(mem, weights):
     assert np.array_equal(crow, np.concatenate([[0], np.cumsum(np.bincount(key // nc, minlength=nc))]))
     assert np.array_equal(ccol, key % nc)
     assert np.array_equal(cw, total.astype(np.float32 if weights == "float" else np.int32))
+
+
+@pytest.mark.parametrize("weights", ["float", "int"])
+def test_rows_at_batch_edges_match_oracle(mem, weights):
+    """Rows of up to, exactly and just above two, four and eight groups of 32 edges, and whole batches with every
+    remainder, in the own-weight, afterburner and inner-connectivity sums of a run."""
+    from oracle import oracle as O
+    degs = [31, 32, 33, 63, 64, 65, 95, 96, 97, 127, 128, 129, 159, 160, 161, 191, 193, 224, 255, 256, 257, 287, 320,
+            352, 383, 385, 449, 511, 512, 513, 1023, 1025]
+    n = 9000
+    rng = np.random.default_rng(5)
+    hubs = np.arange(len(degs)) * 7
+    leaves = np.setdiff1d(np.arange(n), hubs)
+    u = np.concatenate([np.repeat(h, k) for h, k in zip(hubs, degs)])
+    # a hub's leaves come from its own stretch of the ring mostly
+    v = np.concatenate([leaves[(np.arange(k) + i * 270) % len(leaves)] for i, k in enumerate(degs)])
+    ring = np.arange(len(leaves))
+    u = np.concatenate([u, leaves, leaves])
+    v = np.concatenate([v, leaves[(ring + 1) % len(leaves)], leaves[(ring + 2) % len(leaves)]])
+    key = np.unique(np.concatenate([u * n + v, v * n + u]).astype(np.int64))
+    src, col = key // n, (key % n).astype(np.int32)
+    deg = np.bincount(src, minlength=n)
+    assert np.array_equal(deg[hubs], degs)
+    lo, hi = np.minimum(src, col), np.maximum(src, col)
+    _, inv = np.unique(lo * n + hi, return_inverse=True)
+    k = rng.integers(1, 1 << 22, int(inv.max()) + 1)[inv]
+    w = (k * 2.0 ** -22).astype(np.float32) if weights == "float" else (1 + k % 5).astype(np.int32)
+    rowptr = np.concatenate([[0], np.cumsum(deg)]).astype(np.int64)
+    g = pg.weighted_graph(mem, rowptr, col, w, objective=pg.OBJ_WMOD)
+    og = O.Graph(rowptr, col, w, objective=pg.OBJ_WMOD)
+    for seed in (1, 2):
+        cd = pg.get_objective(mem, g, pg.OBJ_WMOD)
+        lab, st = pg.run_clustering(mem, g, cd, method=pg.METHOD_LEIDEN_PLUS, ex_iters=1, seed=seed)
+        lo_, so = O.run_clustering(og, O.ClusterData(og, pg.OBJ_WMOD, 1.0), method=pg.METHOD_LEIDEN_PLUS, ex_iters=1,
+                                   seed=seed)
+        assert np.array_equal(lab, lo_) and st["objective"] == so.objective
+    # a run's FP32 coarse edges are sums rounded to 24 bits
+    rel = 2.0 ** -23 if weights == "float" else 1e-12
+    assert pg.verify_objective(mem, g, lab, pg.OBJ_WMOD)[0] == pytest.approx(st["objective"], rel=rel)
