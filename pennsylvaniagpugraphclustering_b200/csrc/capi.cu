@@ -157,15 +157,18 @@ __global__ void k_validate_offsets(const i64* rowptr, i64 n, i64 nnz, int* bad) 
         if (b < 0 || e < b || e > nnz || (i == 0 && b != 0) || (i == n - 1 && e != nnz)) atomicOr(bad, 1);
     }
 }
-// A warp takes 1,024 consecutive edges, whatever rows they belong to (eight
-// lanes a row read an R-MAT hub's 50,000 columns in 1.3 ms).
-__global__ void __launch_bounds__(256) k_validate_columns(const i64* rowptr, const i32* col, i64 n, i64 nnz, int* bad) {
+// A warp takes `chunk` consecutive edges, whatever rows they belong to (eight
+// lanes a row read an R-MAT hub's 50,000 columns in 1.3 ms): 1,024 where there
+// are enough for all warps, fewer in small graphs (with 1,024 the 117 K edges
+// of a 20,000-vertex graph were 114 warps, 25 us more than eight lanes a row).
+__global__ void __launch_bounds__(256) k_validate_columns(const i64* rowptr, const i32* col, i64 n, i64 nnz, i64 chunk,
+                                                          int* bad) {
     if (*(volatile int*)bad & 1) return;
     const int l = lane_id();
     const i64 gw = (blockIdx.x * (i64)blockDim.x + threadIdx.x) >> 5, nw = ((i64)gridDim.x * blockDim.x) >> 5;
     int found = 0;
-    for (i64 j0 = gw * 1024; j0 < nnz; j0 += nw * 1024) {
-        const i64 j1 = min(nnz, j0 + 1024);
+    for (i64 j0 = gw * chunk; j0 < nnz; j0 += nw * chunk) {
+        const i64 j1 = min(nnz, j0 + chunk);
         i64 jb = j0, u0 = edge_owner(rowptr, n, jb);
         while (jb < j1) {
             const i64 R = u0 + l < n ? rowptr[u0 + l] : (i64)1 << 62;
@@ -201,8 +204,9 @@ void validate_csr_device(Context& c, const i64* rowptr, const i32* col, i64 n, i
                                                                                                            nnz, bad.p);
         PGGC_LAUNCH_CHECK();
         if (nnz > 0) {
-            k_validate_columns<<<(int)std::min<i64>(ceil_div(nnz, 8192), (i64)c.num_sms * 16), 256, 0, c.stream>>>(
-                rowptr, col, n, nnz, bad.p);
+            const i64 chunk = edge_chunk(c, nnz, 32);
+            k_validate_columns<<<(int)std::min<i64>(ceil_div(nnz, 8 * chunk), (i64)c.num_sms * 16), 256, 0, c.stream>>>(
+                rowptr, col, n, nnz, chunk, bad.p);
             PGGC_LAUNCH_CHECK();
         }
     }

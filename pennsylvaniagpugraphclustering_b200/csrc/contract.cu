@@ -6,7 +6,7 @@
 //  2. scans give member offsets and per-coarse-vertex scratch offsets; members
 //     are scattered (counting sort by coarse id) and their degrees prefix-summed
 //     so each coarse vertex owns one flat member-edge list;
-//  3. flattening: one coalesced pass over the CSR, 1,024 edges to a warp,
+//  3. flattening: one coalesced pass over the CSR, up to 1,024 edges to a warp,
 //     writes every edge's coarse key (or -1 inside the coarse vertex: dropped
 //     self-loops, src/contract.cpp:191,209) and weight at its flat position;
 //  4. one pass sorts the rows into buckets; hashed merge of the keys reads each
@@ -65,22 +65,22 @@ __global__ void k_scatter_members(const i32* vcmap, i64 n, i64* cursor, i32* mem
 // Flattening: every fine edge (u, v) is written once, at its position in its
 // coarse row's flat member-edge list (P[memberpos[u]] + rank within u's row),
 // as the coarse key vcmap[v] (-1 for an edge inside the coarse vertex, a
-// self-loop of the coarse graph) and its weight.  A warp takes FL_CHUNK
+// self-loop of the coarse graph) and its weight.  A warp takes `chunk`
 // consecutive edges, whatever rows they belong to (a warp per 32 vertices gave
 // the hubs of an R-MAT graph to a few warps: 12.9 ms for 128 M edges); it holds
 // a window of 32 vertices, and each lane finds its edge's source among them by
 // a 5-step shuffle search of the row offsets.  After this pass the hashing
 // kernels read their rows as contiguous streams.
-constexpr int FL_CHUNK = 1024;
+constexpr int FL_UNROLL = 4;
 
 template <class W>
 __global__ void __launch_bounds__(256) k_flatten(DGraph<W> g, const i32* vcmap, const i64* P, const i64* memberpos,
-                                                 i32* fkey, W* fw) {
+                                                 i32* fkey, W* fw, i64 chunk) {
     const int l = lane_id();
     const i64 gw = (blockIdx.x * (i64)blockDim.x + threadIdx.x) >> 5;
     const i64 nw = ((i64)gridDim.x * blockDim.x) >> 5;
-    for (i64 j00 = gw * FL_CHUNK; j00 < g.nnz; j00 += nw * FL_CHUNK) {
-        const i64 j11 = min(g.nnz, j00 + FL_CHUNK);
+    for (i64 j00 = gw * chunk; j00 < g.nnz; j00 += nw * chunk) {
+        const i64 j11 = min(g.nnz, j00 + chunk);
         i64 jb = j00;
         i64 u0 = edge_owner(g.rowptr, g.n, jb);
         while (jb < j11) {
@@ -93,7 +93,6 @@ __global__ void __launch_bounds__(256) k_flatten(DGraph<W> g, const i32* vcmap, 
             const i64 e1 = min(je, j11);
             // FL_UNROLL groups of 32 edges per iteration: their loads are issued
             // together so that several gathers are in flight per warp
-            constexpr int FL_UNROLL = 4;
             for (i64 j0 = jb; j0 < e1; j0 += 32 * FL_UNROLL) {
                 i32 col[FL_UNROLL];
                 W wv[FL_UNROLL];
@@ -1082,8 +1081,9 @@ std::unique_ptr<Graph<W>> build_coarse_graph(Context& ctx, const Graph<W>& g, co
     WsBuf<i32> fkey(ctx, CS_FKEY, g.nnz);
     W* fw_p = gv.w ? ctx.ws_get<W>(CS_FW, std::max<i64>(g.nnz, 1)) : nullptr;
     if (g.nnz > 0) {
-        int grid = (int)std::min<i64>(ceil_div(ceil_div(g.nnz, FL_CHUNK), 8), (i64)ctx.num_sms * 16);
-        k_flatten<W><<<grid, 256, 0, ctx.stream>>>(gv, vcmap, P.p, memberpos.p, fkey.p, fw_p);
+        const i64 chunk = edge_chunk(ctx, g.nnz, 32 * FL_UNROLL);
+        int grid = (int)std::min<i64>(ceil_div(ceil_div(g.nnz, chunk), 8), (i64)ctx.num_sms * 16);
+        k_flatten<W><<<grid, 256, 0, ctx.stream>>>(gv, vcmap, P.p, memberpos.p, fkey.p, fw_p, chunk);
         PGGC_LAUNCH_CHECK();
     }
     const i64 total_bound = g.nnz;

@@ -224,6 +224,21 @@ def test_contraction_at_the_long_row_limit(mem, weights):
     assert np.array_equal(cw, total.astype(np.float32 if weights == "float" else np.int32))
 
 
+def test_validation_of_chunks_of_1024(mem):
+    """Above 9.7 M edges a warp checks 1,024 of them (fewer in the smaller graphs above)."""
+    d, n = 32, 330000
+    off = np.concatenate([np.arange(-16, 0), np.arange(1, 17)])
+    col = np.sort((np.arange(n)[:, None] + off) % n, axis=1).astype(np.int32).ravel()
+    rowptr = np.arange(n + 1, dtype=np.int64) * d
+    _create(mem, rowptr, col)
+    for j in (0, 1023, 1024, 5 * 1024 * 1024 - 1, len(col) - 1):
+        for fault in (j // d, n, -1):
+            bad = col.copy()
+            bad[j] = fault
+            with pytest.raises(_lib.InvalidArgument):
+                _create(mem, rowptr, bad)
+
+
 @pytest.mark.parametrize("weights", ["float", "int"])
 def test_rows_at_batch_edges_match_oracle(mem, weights):
     """Rows of up to, exactly and just above two, four and eight groups of 32 edges, and whole batches with every
