@@ -805,7 +805,7 @@ pggc_status pggc_build_coarse_graph(pggc_context* ctx, const pggc_graph* g, cons
                 need(nc >= 0 && nc <= gr.n, "nc out of range");
                 In<i32> map(c, vcmap, gr.n, mem_kind);
                 check_labels(c, map.p, gr.n, nc, "vcmap entries must lie in [0, nc)");
-                auto next = build_coarse_graph(c, gr, map.p, nc);
+                auto next = build_coarse_graph(c, gr, map.p, nc, false);
                 coarsen_vtx_w(c, gr, map.p, *next);
                 c.sync();
                 if constexpr (std::is_same<V, double>::value) {

@@ -1040,10 +1040,11 @@ struct WsBuf {
 };
 
 template <class W>
-std::unique_ptr<Graph<W>> build_coarse_graph(Context& ctx, const Graph<W>& g, const i32* vcmap, i64 nc) {
+std::unique_ptr<Graph<W>> build_coarse_graph(Context& ctx, const Graph<W>& g, const i32* vcmap, i64 nc,
+                                             bool next_level) {
     using V = typename Traits<W>::V;
     ProfScope ps(ctx, "contract");
-    if (auto small = build_coarse_small<W>(ctx, g, vcmap, nc)) return small;
+    if (auto small = build_coarse_small<W>(ctx, g, vcmap, nc, next_level)) return small;
     std::optional<ProfScope> phase;  // sub-phases: prep (count .. flatten), hash, place
     phase.emplace(ctx, "contract_prep");
     auto cg = std::make_unique<Graph<W>>();
@@ -1364,8 +1365,8 @@ void coarsen_vtx_w(Context& ctx, const Graph<W>& g, const i32* vcmap, Graph<W>& 
     PGGC_LAUNCH_CHECK();
 }
 
-template std::unique_ptr<Graph<i32>> build_coarse_graph<i32>(Context&, const Graph<i32>&, const i32*, i64);
-template std::unique_ptr<Graph<float>> build_coarse_graph<float>(Context&, const Graph<float>&, const i32*, i64);
+template std::unique_ptr<Graph<i32>> build_coarse_graph<i32>(Context&, const Graph<i32>&, const i32*, i64, bool);
+template std::unique_ptr<Graph<float>> build_coarse_graph<float>(Context&, const Graph<float>&, const i32*, i64, bool);
 template void coarsen_vtx_w<i32>(Context&, const Graph<i32>&, const i32*, Graph<i32>&);
 template void coarsen_vtx_w<float>(Context&, const Graph<float>&, const i32*, Graph<float>&);
 

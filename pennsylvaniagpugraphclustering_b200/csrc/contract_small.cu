@@ -23,6 +23,22 @@ namespace pggc {
 constexpr i64 CS_MATRIX_NC = 1024;
 constexpr int CS_WARP_BOUND = 256;  // member edges of a warp's row (512 table slots)
 constexpr int CS_DENSE = 16384;     // coarse ids of one pass of a block's table
+// Where the one launch is the faster way.  Its lists are made for graphs of even
+// degree: a giant cluster of a skewed graph is one block's, a hub's row eight
+// lanes'.  One launch / the general path, us:
+//   matrix: R-MAT 2,048 vertices 153 / 183; DC-SBM 10,000 (195 K edges, rows up
+//   to 1,557) 161 / 237; star of 14,000 655 / 245 (eight lanes), hence the limit
+//   lists, degrees up to 64: mean degree 6, 47 K edges 121 / 182, 140 K 196 / 219;
+//   mean degree 15, 85 K edges 147 / 187 (FP32 175 / 172), 227 K 234 / 198;
+//   mean degree 30, 108 K edges 149 / 172 (FP32 210 / 176)
+//   lists, skewed: R-MAT 4,096 355 / 219, 16,384 688 / 299; DC-SBM 10,000 557 / 235
+// A level of a run starts on the coarse graph next and would make its ordering,
+// class lists and row sums then (80 us, part of the one launch): lists of any
+// size that lm_small.cuh allows.
+constexpr i64 CS_MATRIX_DEG = 8192;
+constexpr i64 CS_LIST_DEG = 64, CS_LIST_NNZ = 81920;
+constexpr i64 CS_LIST_NNZ_SHORT = 147456;  // mean degree of up to 8
+constexpr i64 CS_WIDE_ROW = 128;    // fine rows that the matrix takes by a warp, not by eight lanes
 
 __device__ __forceinline__ void csum_add(i64* a, i64 x) {
     if (__isShared(a)) shared_add(a, x);
@@ -187,17 +203,32 @@ __global__ void __launch_bounds__(LS_THREADS, 1) k_contract_small(CSmallArgs<W> 
         gang_sync();
         for (i64 base = (i64)gang_warp() * 4; base < n; base += nw * 4) {
             const i64 i = base + grp;
-            if (i >= n) continue;
-            const i64 b = g.rowptr[i], e = g.rowptr[i + 1];
-            const i64 row = (i64)a.vcmap[i] * nc, self = a.vcmap[i];
-#pragma unroll 4
-            for (i64 j = b + r8; j < e; j += 8) {
+            i64 b = 0, e = 0;
+            i32 self = 0;
+            if (i < n) {
+                b = g.rowptr[i];
+                e = g.rowptr[i + 1];
+                self = a.vcmap[i];
+            }
+            auto edge = [&](i64 j, i32 c) {
                 const i32 cv = a.vcmap[g.col[j]];
                 const W x = g.wgt(j);
-                if (cv != self) {
-                    csum_add(&a.oval[row + cv], V(x));
-                    pres[row + cv] = 1;
+                if (cv != c) {
+                    csum_add(&a.oval[(i64)c * nc + cv], V(x));
+                    pres[(i64)c * nc + cv] = 1;
                 }
+            };
+            const bool wide = e - b > CS_WIDE_ROW;
+            if (!wide) {
+#pragma unroll 4
+                for (i64 j = b + r8; j < e; j += 8) edge(j, self);
+            }
+            for (unsigned m = __ballot_sync(FULL, wide && r8 == 0); m; m &= m - 1) {
+                const int from = __ffs(m) - 1;
+                const i64 wb = __shfl_sync(FULL, b, from), we = __shfl_sync(FULL, e, from);
+                const i32 wc = __shfl_sync(FULL, self, from);
+#pragma unroll 4
+                for (i64 j = wb + l; j < we; j += 32) edge(j, wc);
             }
         }
         gang_sync();
@@ -405,14 +436,23 @@ __global__ void __launch_bounds__(LS_THREADS, 1) k_contract_small(CSmallArgs<W> 
 }
 
 template <class W>
-std::unique_ptr<Graph<W>> build_coarse_small(Context& ctx, const Graph<W>& g, const i32* vcmap, i64 nc) {
+std::unique_ptr<Graph<W>> build_coarse_small(Context& ctx, const Graph<W>& g, const i32* vcmap, i64 nc,
+                                             bool next_level) {
     using V = typename Traits<W>::V;
     const i64 n = g.n, nnz = g.nnz;
     if (nc == 0 || n == 0 || ctx.probe_cap != 0) return nullptr;
+    const bool matrix = nc <= CS_MATRIX_NC;
+    {
+        GraphCache& c = *g.cache;
+        std::lock_guard<std::mutex> lk(c.mu);
+        const i64 deg = c.ord_ok ? c.ord.max_deg : -1;  // -1: not known
+        if (matrix ? deg > CS_MATRIX_DEG
+                   : deg < 0 || deg > CS_LIST_DEG || (!next_level && nnz > (nnz <= 8 * n ? CS_LIST_NNZ_SHORT : CS_LIST_NNZ)))
+            return nullptr;
+    }
     const int blocks = gang_blocks(ctx, k_contract_small<W>, small_cluster_blocks(n, nnz));
     if (blocks == 0) return nullptr;
     ProfScope ps(ctx, "contract_small");
-    const bool matrix = nc <= CS_MATRIX_NC;
     const i64 room = std::max<i64>(std::min<i64>(nnz, nc * (nc - 1)), 1);
     auto cg = std::make_unique<Graph<W>>();
     cg->n = nc;
@@ -478,7 +518,8 @@ std::unique_ptr<Graph<W>> build_coarse_small(Context& ctx, const Graph<W>& g, co
     return cg;
 }
 
-template std::unique_ptr<Graph<i32>> build_coarse_small<i32>(Context&, const Graph<i32>&, const i32*, i64);
-template std::unique_ptr<Graph<float>> build_coarse_small<float>(Context&, const Graph<float>&, const i32*, i64);
+template std::unique_ptr<Graph<i32>> build_coarse_small<i32>(Context&, const Graph<i32>&, const i32*, i64,
+                                                                    bool);
+template std::unique_ptr<Graph<float>> build_coarse_small<float>(Context&, const Graph<float>&, const i32*, i64, bool);
 
 }  // namespace pggc

@@ -107,7 +107,8 @@ bool local_move_small(Context& ctx, const Graph<W>& g, const Ordering& ord, i32*
 // build_coarse_graph of a small graph, with its degree ordering, class lists
 // and row sums; null, with nothing done, when the general path has to run it.
 template <class W>
-std::unique_ptr<Graph<W>> build_coarse_small(Context& ctx, const Graph<W>& g, const i32* vcmap, i64 nc);
+std::unique_ptr<Graph<W>> build_coarse_small(Context& ctx, const Graph<W>& g, const i32* vcmap, i64 nc,
+                                             bool next_level);
 
 // workspace slots of the small contraction
 enum ContractSmallSlot : int {

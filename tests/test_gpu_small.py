@@ -345,3 +345,51 @@ def test_size_limits_of_the_one_launch_move(mem, n, d, fits):
         _, want = move()
     for x, y in zip(got, want):
         np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("weights", [None, "int", "float"])
+@pytest.mark.parametrize("n,d,nc,one", [(8000, 10, 1025, True), (8000, 10, 5000, True), (8200, 10, 1025, False),
+                                        (24000, 6, 20000, True), (24600, 6, 1100, False),
+                                        (1200, 64, 1030, True), (1200, 66, 1030, False),   # degree limit of the lists
+                                        (1200, 66, 1024, True)])                           # the matrix has none here
+def test_which_contraction_runs(mem, n, d, nc, one, weights):
+    """Rings of even degree around the limits, one cluster of a third of the vertices: the path, and its rows."""
+    col = np.sort((np.arange(n)[:, None] + np.delete(np.arange(-(d // 2), d // 2 + 1), d // 2)) % n, axis=1).ravel()
+    src = np.repeat(np.arange(n), d)
+    w = None
+    if weights:
+        k = (np.minimum(src, col) * n + np.maximum(src, col)) * 2654435761 % 1000003
+        w = (k % 9 - 2).astype(np.int32) if weights == "int" else ((k + 1) * 2.0 ** -20).astype(np.float32)
+    g = pg.weighted_graph(mem, np.arange(n + 1, dtype=np.int64) * d, col.astype(np.int32), w,
+                          objective=_objective(weights))
+    rng = np.random.default_rng(nc)
+    rest = n - nc
+    m = np.concatenate([np.arange(nc), np.where(rng.random(rest) < 0.33, 0, rng.integers(0, nc, rest))])
+    vcmap = rng.permutation(m).astype(np.int32)
+    # the degrees are known from an earlier move
+    pg.local_move(mem, g, np.arange(n, dtype=np.int32), pg.get_objective(mem, g, _objective(weights)), True)
+    l0 = _lib.lib().pggc_launch_count()
+    got = pg.build_coarse_graph(mem, g, vcmap, nc)
+    launches = _lib.lib().pggc_launch_count() - l0
+    assert (launches <= 4) == one  # label check, contraction, vertex weights
+    with general_path(mem):
+        want = pg.build_coarse_graph(mem, g, vcmap, nc)
+    for a, b in zip(got.to_host(), want.to_host()):
+        assert np.array_equal(a, b)
+
+
+def test_contraction_of_a_skewed_graph_is_general(mem):
+    """A hub's row would be a few lanes' work: 8,193 edges go to the general path also with few clusters."""
+    for leaves, one in ((8192, True), (8193, False)):
+        g = pg.graph_from_edges(mem, leaves + 1, np.zeros(leaves, np.int32), np.arange(1, leaves + 1, dtype=np.int32))
+        vcmap = (np.arange(leaves + 1) % 11).astype(np.int32)
+        pg.generate_orderings(mem, g)
+        pg.local_move(mem, g, np.arange(g.n, dtype=np.int32), pg.get_objective(mem, g, pg.OBJ_MOD), True)
+        l0 = _lib.lib().pggc_launch_count()
+        c = pg.build_coarse_graph(mem, g, vcmap, 11)
+        assert (_lib.lib().pggc_launch_count() - l0 <= 4) == one
+        rowptr, col, w, _ = c.to_host()
+        hub = [(leaves + 1 - k + 10) // 11 for k in range(1, 11)]  # leaves in the other clusters, all joined to vertex 0
+        assert np.array_equal(rowptr, np.concatenate([[0, 10], 10 + np.arange(1, 11)]))
+        assert np.array_equal(col, np.concatenate([np.arange(1, 11), np.zeros(10)]))
+        assert np.array_equal(w, hub + hub)
