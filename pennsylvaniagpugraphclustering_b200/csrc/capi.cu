@@ -247,7 +247,6 @@ std::unique_ptr<Graph<W>> make_graph(Context& ctx, int64_t n, int64_t nnz, const
     }
     row_sums<W>(ctx, *g);
     ctx.sync();
-    g->cache->sums.clear();
     return g;
 }
 
@@ -266,7 +265,6 @@ std::unique_ptr<Graph<i32>> adopt_graph(Context& ctx, i64 n, i64 nnz, DBuf<i64>&
     default_vertex_weights<i32>(ctx, *g, objective);
     row_sums<i32>(ctx, *g);
     ctx.sync();
-    g->cache->sums.clear();
     return g;
 }
 
@@ -807,6 +805,7 @@ pggc_status pggc_build_coarse_graph(pggc_context* ctx, const pggc_graph* g, cons
                 check_labels(c, map.p, gr.n, nc, "vcmap entries must lie in [0, nc)");
                 auto next = build_coarse_graph(c, gr, map.p, nc, false);
                 coarsen_vtx_w(c, gr, map.p, *next);
+                next->cache->shared = true;
                 c.sync();
                 if constexpr (std::is_same<V, double>::value) {
                     cg->kind = PGGC_W_FLOAT32;

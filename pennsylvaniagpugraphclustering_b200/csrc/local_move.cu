@@ -1458,10 +1458,11 @@ __global__ void k_row_degrees(const i64* rowptr, i64 n, V* out) {
 }
 
 // Kept with the graph.  The kernels that fill them are queued and not waited
-// for: a coarse graph may get its sums from one of several jobs that share it,
-// so a call on another stream waits for the mark that the first one left.
-// (The units are values that tables are built on: read too early they turn
-// fractional weights into whole numbers.)
+// for.  Graphs are handed out with their sums complete, and a run's levels
+// belong to one stream; only a coarse graph that the caller asked for may get
+// them from one of several jobs that share it, and the other streams then wait
+// for the mark that the first one left.  (The units are values that tables are
+// built on: read too early they turn fractional weights into whole numbers.)
 template <class W>
 const typename Traits<W>::V* row_sums(Context& ctx, const Graph<W>& g) {
     using V = typename Traits<W>::V;
@@ -1495,7 +1496,7 @@ const typename Traits<W>::V* row_sums(Context& ctx, const Graph<W>& g) {
             PGGC_LAUNCH_CHECK();
         }
     }
-    c.sums.set(ctx);
+    if (c.shared) c.sums.set(ctx);
     g.units = std::move(units);
     g.rsum = std::move(sums);
     return g.rsum.p;
