@@ -214,7 +214,8 @@ bool local_move_small(Context& ctx, const Graph<W>& g, const Ordering& ord, i32*
     using V = typename Traits<W>::V;
     const i64 n = g.n;
     const bool long_rows = g.nnz >= 64 * n;
-    const bool fits = long_rows ? g.nnz <= LS_MOVE_NNZ_LONG : g.nnz + 4 * n <= LS_MOVE_SIZE;
+    const bool fits =
+        long_rows ? g.nnz <= LS_MOVE_NNZ_LONG : g.nnz <= LS_MOVE_NNZ && g.nnz + 4 * n <= LS_MOVE_SIZE;
     const int want = fits ? small_cluster_blocks(n, g.nnz) : 0;
     auto& F = ctx.filt;
     const bool filt_on = F.mode != 0 && !strict;

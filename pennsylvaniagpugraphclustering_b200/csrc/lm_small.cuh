@@ -9,19 +9,23 @@ namespace pggc {
 // Above these a launch per step over the whole GPU is the faster way: the work
 // on the cluster's 16 SMs grows with the edges while the launches do not.
 // Local moves have the lower limits (their steps cover the GPU in 7 launches a
-// sweep, contraction and refinement take 25 to 30), on the edges plus what a
-// vertex costs beside its edges, about four of them.  Six sweeps here and with
-// a launch per step, us (planted partitions / power-law degrees):
+// sweep, contraction and refinement take 25 to 30), on the edges and on the
+// edges plus what a vertex costs beside them, about four.  Six sweeps here and
+// with a launch per step, us (planted partitions / power-law degrees):
 //   mean degree 4:    49 K edges 371, 421 / 496, 499; 127 K 667, 468 / 938, 520
 //   mean degree 8:    68 K edges 377, 412 / 511, 516; 155 K 559, 455 / 941, 532
 //   mean degree 15:   57 K edges 329, 441; 104 K 447, 444 / 598, 599; 227 K 704, 464
 //   mean degree 30:   81 K edges 370, 459 / 497, 603; 144 K 531, 469 / 805, 691
+// One run at a time that would be 115 K edges and vertices; in a batch a launch
+// and no round trip a sweep is worth more (32 graphs of 6,000 to 12,000 vertices
+// of 14 edges on 4 streams: 21.9 ms with that limit, 21.0 ms with these).
 // Long rows go further, a warp or block has enough to do in each:
 //   mean degree 55:  133 K edges 459, 451;  75: 158 K 362, 386 (FP32 weights 520,
 //   512);  94: 170 K 311, 369 (446, 490);  136: 130 K 189, 307 (335, 472)
 constexpr i64 LS_MAX_N = 32768;
 constexpr i64 LS_MAX_NNZ = 262144;
-constexpr i64 LS_MOVE_SIZE = 114688;      // edges plus four a vertex
+constexpr i64 LS_MOVE_NNZ = 131072;
+constexpr i64 LS_MOVE_SIZE = 163840;      // edges plus four a vertex
 constexpr i64 LS_MOVE_NNZ_LONG = 196608;  // edges, at a mean degree of 64 or more
 constexpr i64 LS_MAX_LABELS = 131072;
 

@@ -322,8 +322,8 @@ def test_filtered_moves(mem, form, weights, net):
     assert evaluated > 0 and skipped > 0
 
 
-@pytest.mark.parametrize("n,d,fits", [(8192, 10, True), (8193, 10, False),    # edges plus four a vertex: 114,688
-                                      (1737, 62, True), (1738, 62, False),
+@pytest.mark.parametrize("n,d,fits", [(11702, 10, True), (11703, 10, False),  # edges plus four a vertex: 163,840
+                                      (2114, 62, True), (2115, 62, False),    # 131,072 edges
                                       (3072, 64, True), (3073, 64, False)])   # long rows: 196,608 edges
 def test_size_limits_of_the_one_launch_move(mem, n, d, fits):
     """Rings where every vertex has d neighbours, at the limits and just above: the path that runs, and its answer."""
