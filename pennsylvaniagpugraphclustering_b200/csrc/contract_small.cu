@@ -33,11 +33,15 @@ constexpr int CS_DENSE = 16384;     // coarse ids of one pass of a block's table
 //   mean degree 30, 108 K edges 149 / 172 (FP32 210 / 176)
 //   lists, skewed: R-MAT 4,096 355 / 219, 16,384 688 / 299; DC-SBM 10,000 557 / 235
 // A level of a run starts on the coarse graph next and would make its ordering,
-// class lists and row sums then (80 us, part of the one launch): lists of any
-// size that lm_small.cuh allows.
+// class lists and row sums then (80 us, part of the one launch): any size that
+// lm_small.cuh allows and degrees up to 1,024 (whole runs with 64 / 4,096 there:
+// R-MAT 8,192 3,490 / 3,880 us, 16,384 3,360 / 3,640, planted partition of
+// 16,000 1,265 / 1,240, DC-SBM 10,000 2,450 / 2,350; a batch of 46 planted
+// partitions 1.5 % slower with 64).
 constexpr i64 CS_MATRIX_DEG = 8192;
 constexpr i64 CS_LIST_DEG = 64, CS_LIST_NNZ = 81920;
 constexpr i64 CS_LIST_NNZ_SHORT = 147456;  // mean degree of up to 8
+constexpr i64 CS_LIST_DEG_RUN = 1024;
 constexpr i64 CS_WIDE_ROW = 128;    // fine rows that the matrix takes by a warp, not by eight lanes
 
 __device__ __forceinline__ void csum_add(i64* a, i64 x) {
@@ -446,8 +450,11 @@ std::unique_ptr<Graph<W>> build_coarse_small(Context& ctx, const Graph<W>& g, co
         GraphCache& c = *g.cache;
         std::lock_guard<std::mutex> lk(c.mu);
         const i64 deg = c.ord_ok ? c.ord.max_deg : -1;  // -1: not known
-        if (matrix ? deg > CS_MATRIX_DEG
-                   : deg < 0 || deg > CS_LIST_DEG || (!next_level && nnz > (nnz <= 8 * n ? CS_LIST_NNZ_SHORT : CS_LIST_NNZ)))
+        const bool fits = matrix       ? deg <= CS_MATRIX_DEG
+                          : next_level ? deg >= 0 && deg <= CS_LIST_DEG_RUN
+                                       : deg >= 0 && deg <= CS_LIST_DEG &&
+                                             nnz <= (nnz <= 8 * n ? CS_LIST_NNZ_SHORT : CS_LIST_NNZ);
+        if (!fits)
             return nullptr;
     }
     const int blocks = gang_blocks(ctx, k_contract_small<W>, small_cluster_blocks(n, nnz));
